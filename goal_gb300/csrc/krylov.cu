@@ -11,6 +11,7 @@
 
 #include <cuda_fp16.h>
 
+#include <mutex>
 #include <type_traits>
 
 namespace goal {
@@ -21,7 +22,7 @@ struct GState {
   int j;        // completed Arnoldi columns in this cycle
   int done;     // 1: converged, broke down or restart length reached
   int reorth;   // second Gram-Schmidt pass needed for the current column
-  int pad;
+  int pad;      // 1: a grid barrier of the persistent cycle ran out of its limit
   double wb2;   // |w|^2 before orthogonalization
   double res;   // |g[j]| residual estimate
   double beta;  // initial residual norm of the cycle
@@ -76,6 +77,7 @@ __device__ __forceinline__ C thread_partial_sum(const C* __restrict__ p, int n) 
 __device__ __forceinline__ float c_hypot(float a, float b) { return hypotf(a, b); }
 
 constexpr int kMaxM = 256;
+constexpr int kCtl = 4;  // words of Krylov::ctl
 constexpr int kDotChunk = 8;
 // Gram-Schmidt passes: the FP64 outer basis gets the conditional second pass;
 // the fixed-length FP32 inner solve is only a preconditioner of the flexible
@@ -933,16 +935,23 @@ __global__ void k_inner_blocks(int N, const double* __restrict__ Dinv, const dou
   }
 }
 
+#include "krylov_coop.cuh"
+
 int spmv_grid(int N) { return grid_for((long long)N * 4, 256, kSMs * 16); }
 int vec_grid(long long n) { return grid_for(n, 256, kSMs * 8); }
-// Rows per thread of the orthogonalization kernels. FP64: always the longest
-// slab, because the per-block reductions cost FP64 instructions (measured on
-// the 530k-dof nested adjoint: 141 us per multidot pass with 2 rows per thread
-// against 64 us with 8). FP32: enough blocks for about eight per SM, at least
+// Rows per thread of the orthogonalization kernels. FP64: the longest slab,
+// because the per-block reductions cost FP64 instructions (measured on the
+// 530k-dof nested adjoint: 141 us per multidot pass with 2 rows per thread
+// against 64 us with 8), unless shorter ones still leave SMs without a block.
+// FP32: enough blocks for about eight per SM, at least
 // two and at most kMaxRows rows per thread.
 template <typename T>
 int slab_rows(long long n) {
-  if (!std::is_same<T, float>::value) return kMaxRows;
+  if (!std::is_same<T, float>::value) {
+    int r = 1;
+    while (r < kMaxRows && n > 256ll * r * kSMs) r *= 2;
+    return r;
+  }
   const long long target = 8ll * kSMs * 256;
   int r = 2;
   while (r < kMaxRows && n >= 2ll * r * target) r *= 2;
@@ -981,6 +990,7 @@ void Krylov::reserve(int n_, int m_, int mi_, int precision, int nnzb) {
   need(scal, 64);
   need(flag, 8);
   need(dots, kMaxM + 2);
+  need(ctl, kCtl);
   if (has_inner_solve(precision)) {
     const size_t nb = nn * (mi_ + 1);
     if (precision == PREC_MIXED) need(V16, nb);
@@ -1158,6 +1168,78 @@ struct StepGraph {
 
 namespace {
 
+// How a persistent cycle (k_gmres_coop) of N nodes is laid out: nodes per CTA
+// and CTAs, one CTA per SM at most.
+struct CoopPlan {
+  int chunk = 0, grid = 0;
+};
+
+struct CoopDevice {
+  int sms = 0, smem = 0;
+};
+const CoopDevice& coop_device() {
+  constexpr int kDevs = 64;
+  static CoopDevice known[kDevs];
+  static std::mutex guard;
+  int dev = 0;
+  GOAL_CUDA(cudaGetDevice(&dev));
+  GOAL_REQUIRE(dev >= 0 && dev < kDevs, GOAL_ERR_CUDA, "device number out of range");
+  std::lock_guard<std::mutex> lock(guard);
+  CoopDevice& d = known[dev];
+  if (!d.sms) {
+    int coop = 0, optin = 0, sms = 0;
+    GOAL_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    GOAL_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    GOAL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    GOAL_REQUIRE(coop, GOAL_ERR_CUDA, "cooperative launches are not available");
+    d.smem = optin - 512;  // the kernel's static shared memory stays below this
+    d.sms = std::min(sms, kCoopThreads);  // a thread polls one CTA's flag
+  }
+  return d;
+}
+
+// The persistent cycle wins while an Arnoldi step is bound by its launches and
+// its few blocks; past some 800 nodes to an SM the separate kernels, with more
+// threads in flight on the matrix and basis streams, are as fast. Whole solves
+// to 1e-12, ms, kernels -> persistent: FP64 343 nodes 26.5 -> 4.4, 9k 269 ->
+// 69, 24k 651 -> 261; binary16 inner 5k 28.0 -> 14.6, 36k 58 -> 36, 69k 88.5
+// -> 61.6, 118k 145 -> 126, 185k 230 -> 245 (learned 183 -> 247).
+// At least 8 nodes to a CTA: a warp of rows.
+constexpr int kCoopMinNodes = 8;
+constexpr int kCoopNodesPerSm = 800;
+
+bool coop_plan(int N, CoopPlan& p) {
+  const CoopDevice& d = coop_device();
+  if (N > kCoopNodesPerSm * d.sms) return false;
+  p.chunk = std::max(kCoopMinNodes, (N + 8 * d.sms - 1) / (8 * d.sms) * 8);
+  p.grid = (N + p.chunk - 1) / p.chunk;
+  return true;
+}
+
+template <typename T, typename TA, typename TV>
+void launch_coop(const CoopPlan& p, CoopArgs<T, TA, TV> a, int nnzb, cudaStream_t s) {
+  const CoopDevice& d = coop_device();
+  const size_t cap = 4 * (size_t)p.chunk, most = (size_t)d.smem;
+  // w, t, h, coefficients, scales, rotations, the reduction buffer, row pointers
+  const size_t fixed = 2 * sizeof(T) * cap + 12 * sizeof(T) * (size_t)(a.m + 2) + sizeof(T) * kCoopRed +
+                       sizeof(int) * (p.chunk + 1) + 640;
+  GOAL_REQUIRE(fixed <= most, GOAL_ERR_CAPACITY, "persistent cycle: rows per CTA exceed shared memory");
+  const size_t blocks = (a.Bc ? 2 : 1) * sizeof(T) * 4 * cap, basis = sizeof(TV) * (cap + 32) * (a.m + 1);
+  const size_t matrix = (size_t)(1.05 * p.chunk * nnzb / a.N) * (16 * sizeof(TA) + sizeof(int));
+  // Shared memory for the basis and the matrix rows when both fit; what is
+  // left out is read through L1, which is larger the less shared memory is asked for
+  size_t smem = fixed + blocks + 256;
+  if (smem + basis + matrix <= most) smem = most;
+  else if (smem + basis <= most / 2) smem += basis;
+  a.chunk = p.chunk;
+  a.smem_bytes = (int)std::min(smem, most);
+  const void* kernel = (const void*)k_gmres_coop<T, TA, TV>;
+  GOAL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem));
+  void* args[] = {&a};
+  GOAL_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(p.grid), dim3(kCoopThreads + 32), args, (size_t)a.smem_bytes, s));
+  GOAL_CHECK_LAUNCH();
+}
+
 // The inner solve's arrays for one storage / arithmetic combination: matrix
 // (TA), basis (TV), work vectors, block-Jacobi blocks and the small Hessenberg
 // state in the arithmetic type T (FP32 state lives in the FP64 buffers
@@ -1218,6 +1300,33 @@ void issue_inner(const BsrView& A, long long n, int mi, bool sweep2, GState* st,
   const int N = A.num_nodes;
   const int nbx = vec_grid(n);
   cudaStream_t s = K.stream;
+  CoopPlan plan;
+  if (coop_plan(N, plan)) {
+    CoopArgs<T, TA, TV> a{};
+    a.N = N;
+    a.m = mi;
+    a.brow_ptr = A.brow_ptr;
+    a.bcol = A.bcol;
+    a.A = in.A;
+    a.Dinv = in.Dinv;
+    a.Bc = sweep2 ? in.Bc : nullptr;
+    a.V = in.V;
+    a.z1 = in.r;
+    a.z2 = in.t;
+    a.part1 = in.red;
+    a.part2 = in.red + (size_t)(kMaxM + 2) * plan.grid;
+    a.partn = a.part2 + (size_t)(kMaxM + 2) * plan.grid;
+    a.H = in.H;
+    a.y = in.y;
+    a.ctl = K.ctl.ptr;
+    a.src = K.V.ptr;
+    a.sd = K.sd.ptr;
+    a.dst = K.Z.ptr;
+    a.st = st;
+    a.inner = 1;
+    launch_coop(plan, a, A.nnzb, s);
+    return;
+  }
   k_col_to_inner<T><<<nbx, 256, 0, s>>>(n, K.V.ptr, n, st, K.sd.ptr, in.r);
   GOAL_CHECK_LAUNCH();
   k_norm2_part<T><<<nbx, 256, 0, s>>>(n, in.r, in.red);
@@ -1286,6 +1395,8 @@ SolveStats fgmres(const BsrView& A, const double* vals, const double* b, double*
   GState* st = reinterpret_cast<GState*>(K.scal.ptr);         // outer state
   GState* sti = reinterpret_cast<GState*>(K.scal.ptr + 24);   // inner state
   double* dots = K.dots.ptr;
+  GOAL_CUDA(cudaMemsetAsync(K.ctl.ptr, 0, sizeof(unsigned) * kCtl, s));
+  GOAL_CUDA(cudaMemsetAsync(st, 0, sizeof(GState), s));
 
   const double bnorm = read_norm(n, b, K);
   const double tol_abs = p.tolerance * (bnorm > 0.0 ? bnorm : 1.0);
@@ -1330,7 +1441,42 @@ SolveStats fgmres(const BsrView& A, const double* vals, const double* b, double*
   StepGraph step_graph;
   const int batch = mixed ? 1 : 4;
 
+  CoopPlan plan;
+  const bool coop = !mixed && coop_plan(N, plan);
   while (beta > tol_abs && out.iters < p.max_iters) {
+    const int steps = std::min(m, p.max_iters - out.iters);
+    int done_steps = 0;
+    const long long extra = sweep2 ? 1 : 0;
+    if (coop) {  // the whole cycle in one kernel, x += M^-1 V y
+      CoopArgs<double, double, double> a{};
+      a.N = N;
+      a.m = steps;
+      a.two_pass = 1;
+      a.tol_abs = tol_abs;
+      a.brow_ptr = A.brow_ptr;
+      a.bcol = A.bcol;
+      a.A = vals;
+      a.Dinv = K.Dinv.ptr;
+      a.Bc = sweep2 ? K.Bc.ptr : nullptr;
+      a.V = K.V.ptr;
+      a.z1 = K.Z.ptr;
+      a.z2 = K.w.ptr;
+      a.part1 = K.red.ptr;
+      a.part2 = a.part1 + (size_t)(kMaxM + 2) * plan.grid;
+      a.partn = a.part2 + (size_t)(kMaxM + 2) * plan.grid;
+      a.H = K.H.ptr;
+      a.y = K.y.ptr;
+      a.ctl = K.ctl.ptr;
+      a.src = K.r.ptr;
+      a.dst = x;
+      a.st = st;
+      launch_coop(plan, a, A.nnzb, s);
+      GOAL_CUDA(cudaMemcpyAsync(K.h_scal, K.scal.ptr, sizeof(GState), cudaMemcpyDeviceToHost, s));
+      GOAL_CUDA(cudaStreamSynchronize(s));
+      const GState* hs = reinterpret_cast<const GState*>(K.h_scal);
+      GOAL_REQUIRE(!hs->pad, GOAL_ERR_SOLVER, "fgmres: a grid barrier did not complete");
+      done_steps = hs->j;
+    } else {
     // start a cycle: V_0 = r / beta
     k_norm2_part<double><<<nbx, 256, 0, s>>>(n, K.r.ptr, K.red.ptr);
     GOAL_CHECK_LAUNCH();
@@ -1338,9 +1484,7 @@ SolveStats fgmres(const BsrView& A, const double* vals, const double* b, double*
     GOAL_CHECK_LAUNCH();
     k_scale_into<double, double><<<nbx, 256, 0, s>>>(n, K.r.ptr, st, K.V.ptr);
     GOAL_CHECK_LAUNCH();
-    const int steps = std::min(m, p.max_iters - out.iters);
     if (!step_graph.exec) step_graph.capture(s, issue_step);
-    int done_steps = 0;
     for (int step = 0; step < steps;) {
       const int k = std::min(batch, steps - step);
       for (int q = 0; q < k; ++q) step_graph.launch(s);
@@ -1348,10 +1492,15 @@ SolveStats fgmres(const BsrView& A, const double* vals, const double* b, double*
       GOAL_CUDA(cudaMemcpyAsync(K.h_scal, K.scal.ptr, sizeof(GState), cudaMemcpyDeviceToHost, s));
       GOAL_CUDA(cudaStreamSynchronize(s));
       const GState* hs = reinterpret_cast<const GState*>(K.h_scal);
+      GOAL_REQUIRE(!hs->pad, GOAL_ERR_SOLVER, "fgmres: a grid barrier did not complete");
       done_steps = hs->j;
       if (hs->done) break;
     }
-    const long long extra = sweep2 ? 1 : 0;
+    k_backsolve<double><<<1, 32, 0, s>>>(st, K.H.ptr, m + 1, K.g.ptr, K.y.ptr);
+    GOAL_CHECK_LAUNCH();
+    k_combine<double, double><<<nbx, 256, 0, s>>>(n, K.Z.ptr, n, K.y.ptr, st, x, 0);
+    GOAL_CHECK_LAUNCH();
+    }
     if (mixed) {
       out.inner_iters += (long long)mi * done_steps;
       out.spmv32 += (long long)done_steps * (mi * (1 + extra) + extra);
@@ -1360,10 +1509,6 @@ SolveStats fgmres(const BsrView& A, const double* vals, const double* b, double*
       out.spmv64 += (long long)done_steps * (1 + extra);
     }
     out.iters += done_steps;
-    k_backsolve<double><<<1, 32, 0, s>>>(st, K.H.ptr, m + 1, K.g.ptr, K.y.ptr);
-    GOAL_CHECK_LAUNCH();
-    k_combine<double, double><<<nbx, 256, 0, s>>>(n, K.Z.ptr, n, K.y.ptr, st, x, 0);
-    GOAL_CHECK_LAUNCH();
     k_spmv<double, double, true><<<spmv_grid(N), 256, 0, s>>>(N, A.brow_ptr, A.bcol, vals, x, b, K.r.ptr);
     GOAL_CHECK_LAUNCH();
     out.spmv64++;

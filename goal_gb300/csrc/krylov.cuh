@@ -81,6 +81,7 @@ struct Krylov {
   DevBuf<double> Bc;
   DevBuf<float> Bc32;
   DevBuf<int> flag;
+  DevBuf<unsigned> ctl;      // grid barrier and results of a persistent cycle
   double* h_scal = nullptr;  // pinned host mirror of a few scalars
   ~Krylov();
   void reserve(int n_, int m_, int mi_, int precision, int nnzb);
