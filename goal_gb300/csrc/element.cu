@@ -38,6 +38,9 @@
 //   K^pu_{a,bk} = V [ h_bk (tau J w_a - (J+1/J)/8) - tau J e_ab v_k - tau J w_b h_ak ]
 //   K^pp_{ab}   = V [ 1/(16 kappa) + tau J e_ab ]
 // with v = H grad p, w_a = v.h_a, e_ab = h_a.h_b.
+#include <type_traits>
+
+#include "fixed.cuh"
 #include "mechanics.cuh"
 
 namespace goal {
@@ -124,26 +127,22 @@ __device__ bool exp_traceless_sym(const double A[3][3], double out[3][3]) {
   return ok;
 }
 
-// BUF: element outputs go to the per-element buffer (phase 1 of the two-phase
-// assembly) instead of being accumulated in place by one colour at a time.
-// DSUM (with BUF): of the four diagonal element blocks (a, a) only column 3
-// (K^up_a, K^pp_aa) is formed and stored, packed in the block's first four
-// slots. The u columns of a matrix row sum to zero over the row's blocks (the
-// gradients of a linear tet's shape functions sum to zero, and every u column
-// of K^uu and K^pu is linear in them), so k_gather_diag forms the diagonal
-// blocks' u columns as negated sums of the off-diagonal blocks.
-template <int MODEL, int MODE, bool JAC, bool ERR, bool BUF, bool DSUM = false>
-__global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
-  const int s = a.begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= a.end) return;
-  const int E = a.d.num_elems;
+// What the integration point of an element gives the residual and the tangent.
+struct Point {
+  double V, inv_kappa, tau_coef, pp_coef;
+  double un[4][3], pval, gp[3];           // nodal displacements, pressure and its gradient
+  double J, Jinv, H[3][3], C[6], FC[3][3];
+  double alpha, Ic3, s[6];                // s: trial deviatoric Kirchhoff stress xx yy zz xy yz xz
+  double gamma, smag, mubar, fyield, k0, cc, kh, rsmag, rcc;
+  bool plastic;
+  double sg[3][3];                        // Cauchy stress after Mixed
+};
 
-  int v[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) v[q] = __ldg(a.d.tets + q * E + s);
-  double G[4][3];
-#pragma unroll
-  for (int q = 0; q < 12; ++q) G[q / 3][q % 3] = __ldg(a.d.grads + q * E + s);
+// Gather, kinematics, constitutive model with its state writes, and Mixed.
+template <int MODEL>
+__device__ __forceinline__ void eval_point(const ElemArgs& a, int s, const int (&v)[4], const double (&G)[4][3],
+                                           Point& p) {
+  const int E = a.d.num_elems;
   const double V = __ldg(a.d.vol + s);
   const int es = __ldg(a.d.elem_set + s);
   const double* mrow = a.mats + kMatStride * es;
@@ -304,6 +303,53 @@ __global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
 #pragma unroll
     for (int q = 0; q < 9; ++q) a.sigma[q * E + s] = sg[q / 3][q % 3];
   }
+
+
+  p.V = V; p.inv_kappa = inv_kappa; p.tau_coef = tau_coef; p.pp_coef = pp_coef;
+  p.pval = pval; p.J = J; p.Jinv = Jinv; p.alpha = alpha; p.Ic3 = Ic3;
+  p.s[0] = s00; p.s[1] = s11; p.s[2] = s22; p.s[3] = s01; p.s[4] = s12; p.s[5] = s02;
+  p.gamma = gamma; p.smag = smag; p.mubar = mubar; p.fyield = fyield; p.k0 = k0; p.cc = cc; p.kh = kh;
+  p.rsmag = rsmag; p.rcc = rcc; p.plastic = plastic;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    p.gp[i] = gp[i];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) { p.H[i][j] = H[i][j]; p.FC[i][j] = FC[i][j]; p.sg[i][j] = sg[i][j]; }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) p.un[q][i] = un[q][i];
+  }
+#pragma unroll
+  for (int q = 0; q < 6; ++q) p.C[q] = C[q];
+}
+
+// BUF: element outputs go to the per-element buffer (phase 1 of the two-phase
+// assembly) instead of being accumulated in place by one colour at a time.
+template <int MODEL, int MODE, bool JAC, bool ERR, bool BUF>
+__global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
+  const int s = a.begin + blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= a.end) return;
+  const int E = a.d.num_elems;
+
+  int v[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = __ldg(a.d.tets + q * E + s);
+  double G[4][3];
+#pragma unroll
+  for (int q = 0; q < 12; ++q) G[q / 3][q % 3] = __ldg(a.d.grads + q * E + s);
+  Point pt;
+  eval_point<MODEL>(a, s, v, G, pt);
+  const double V = pt.V, inv_kappa = pt.inv_kappa, tau_coef = pt.tau_coef, pp_coef = pt.pp_coef;
+  const double pval = pt.pval, J = pt.J, Jinv = pt.Jinv, alpha = pt.alpha, Ic3 = pt.Ic3;
+  const double s00 = pt.s[0], s11 = pt.s[1], s22 = pt.s[2], s01 = pt.s[3], s12 = pt.s[4], s02 = pt.s[5];
+  const double gamma = pt.gamma, smag = pt.smag, mubar = pt.mubar, fyield = pt.fyield, k0 = pt.k0, cc = pt.cc;
+  const double kh = pt.kh, rsmag = pt.rsmag, rcc = pt.rcc;
+  const bool plastic = pt.plastic;
+  const double(&H)[3][3] = pt.H;
+  const double(&FC)[3][3] = pt.FC;
+  const double(&sg)[3][3] = pt.sg;
+  const double(&C)[6] = pt.C;
+  const double(&gp)[3] = pt.gp;
+  const double(&un)[4][3] = pt.un;
 
   // h_a = H G_a
   double hv[4][3];
@@ -503,7 +549,6 @@ __global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
 #pragma unroll
   for (int b = 0; b < 4; ++b) twv[b] = a.stab ? tJV * wv[b] : 0.0;
   const double tJVs = a.stab ? tJV : 0.0;
-  const unsigned fm = (!BUF && a.overwrite) ? __ldg(a.d.first + s) : 0u;
   // ga V C G_a and Z_a = zs h_a
   double CG[4][3], Zv[4][3];
 #pragma unroll
@@ -518,6 +563,7 @@ __global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) Zv[ai][k] = zs * hv[ai][k];
   }
+  const unsigned fm = (!BUF && a.overwrite) ? __ldg(a.d.first + s) : 0u;
   // Element block (ai, b) from Pc[i][k] = h_bi Z_ak + c_ab d_ik (TP: Pc
   // transposed), written to the element buffer or accumulated into the matrix.
   auto block = [&](int ai, int b, const double (&Pc)[3][3], bool TP, double eab) {
@@ -572,21 +618,425 @@ __global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
 #pragma unroll
   for (int ai = 0; ai < 4; ++ai) {
     const double eaa = hv[ai][0] * hv[ai][0] + hv[ai][1] * hv[ai][1] + hv[ai][2] * hv[ai][2];
-    if constexpr (DSUM) {
-      // column 3 only: the u columns come from the row sums in the gather
-      st4(a.ebuf + (size_t)(s - a.ebase) * a.estride + 16 + 16 * (5 * ai), upf * hv[ai][0], upf * hv[ai][1],
-          upf * hv[ai][2], fma(tJVs, eaa, ppc));
-    } else {
-      const double caa = fma(CG[ai][0], G[ai][0], fma(CG[ai][1], G[ai][1], CG[ai][2] * G[ai][2]));
-      double Pc[3][3];
+    const double caa = fma(CG[ai][0], G[ai][0], fma(CG[ai][1], G[ai][1], CG[ai][2] * G[ai][2]));
+    double Pc[3][3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int k = 0; k < 3; ++k) Pc[i][k] = (i == k) ? fma(hv[ai][i], Zv[ai][k], caa) : hv[ai][i] * Zv[ai][k];
-      block(ai, ai, Pc, false, eaa);
-    }
+      for (int k = 0; k < 3; ++k) Pc[i][k] = (i == k) ? fma(hv[ai][i], Zv[ai][k], caa) : hv[ai][i] * Zv[ai][k];
+    block(ai, ai, Pc, false, eaa);
   }
   }  // JAC
+}
+
+// ------------------------------------------------------------------ fixed-point element phase
+// Element record of the default Jacobian assembly, kRecord 8-byte words:
+//   [0, 16)    R (FP64)
+//   [16, 32)   per block (a, b) four 16-bit exponents: of K^uu, K^up, K^pu, K^pp
+//   [32, 48)   column 3 (K^up_a, K^pp_aa) of the diagonal blocks
+//   [48, 240)  the twelve off-diagonal blocks, row-major
+// with every block entry S 2^x in the fixed point of fixed.cuh.
+constexpr int kRecord = 240;
+constexpr int kRecExp = 16, kRecDiag = 32, kRecOff = 48;
+__device__ __forceinline__ int off_index(int a, int b) { return 3 * a + b - (b > a ? 1 : 0); }
+
+// Residual and tangent of one element per thread into its record, for both
+// Jacobian modes (the gather transposes).
+//
+// The 144 entries of the off-diagonal element blocks are sums of two or three
+// products and took 450 of the 1,014 FP64 instructions per element; here they
+// are formed in fixed point on the integer pipes (see fixed.cuh), and so are
+// the vectors that enter them (m, q, n, X, Y, Z: another 210). The blocks come
+// in pairs as c_ab, e_ab and h_b Z_a are shared by (a, b) and (b, a).
+//
+// Of the diagonal element blocks only column 3 is formed: the u columns of a
+// matrix row sum to zero over the row's blocks (the gradients of a linear
+// tet's shape functions sum to zero, and every u column of K^uu and K^pu is
+// linear in them), so k_gather_rows forms the diagonal blocks' u columns as
+// negated sums of the off-diagonal blocks.
+//
+// The factors wait in shared memory (a column of kFixSlots words per thread)
+// and the loops over nodes and pairs are not unrolled: unrolled, the kernel
+// was 12,800 instructions long and waited for instruction fetches 43% of the
+// time. J2 at 384,000 elements: 740 us in FP64 throughout, 1,208 unrolled, 498
+// with FP64 vectors m, q, n, X, Y, Z, now 432 (neo-Hookean 327). What bounds
+// it is latency at three warps per scheduler (registers and shared memory);
+// the FP64 pipe is 48% busy.
+constexpr int kFixThreads = 128;
+constexpr int kFixC = 60, kFixW = 66, kFixSlots = 70;  // factors of h, q, X, Y, Z; c_ab; w_a
+
+template <int MODEL>
+__global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
+  extern __shared__ long long fix_slots[];
+  const int s = a.begin + blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= a.end) return;
+  const int E = a.d.num_elems;
+  long long* slot = fix_slots + threadIdx.x;
+  auto factor = [&](int i) {
+    const long long r = slot[i * kFixThreads];
+    Fx f;
+    f.lo = (int)r;
+    f.hi = (int)(r >> 32);
+    return f;
+  };
+  auto put_factor = [&](int i, const Fx& f) {
+    slot[i * kFixThreads] = ((long long)f.hi << 32) | (unsigned)f.lo;
+  };
+  auto at = [](int v, int n, int k) { return 12 * v + 3 * n + k; };  // v: h q X Y Z
+  double* rec_r = a.ebuf + (size_t)(s - a.ebase) * kRecord;
+  long long* rec = reinterpret_cast<long long*>(rec_r);
+
+  int v[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = __ldg(a.d.tets + q * E + s);
+  Point pt;
+  {
+    double G[4][3];
+#pragma unroll
+    for (int q = 0; q < 12; ++q) G[q / 3][q % 3] = __ldg(a.d.grads + q * E + s);
+    eval_point<MODEL>(a, s, v, G, pt);
+  }
+  const double V = pt.V, J = pt.J, Jinv = pt.Jinv, alpha = pt.alpha, Ic3 = pt.Ic3, gamma = pt.gamma;
+  const double(&H)[3][3] = pt.H;
+  const double(&FC)[3][3] = pt.FC;
+
+  // residual coefficients, as in k_elem
+  double vv[3], TV[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    vv[i] = H[i][0] * pt.gp[0] + H[i][1] * pt.gp[1] + H[i][2] * pt.gp[2];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) TV[i][j] = V * (J * pt.sg[i][j]);
+  }
+  double tau = 0.0;
+  if (a.stab) {
+    const double hh = __ldg(a.d.h + s);
+    tau = pt.tau_coef * (hh * hh);
+  }
+  const double tauJ = tau * J;
+  const double rp0 = ((pt.pval * pt.inv_kappa) - 0.5 * (J - Jinv)) * 0.25 * V;
+  const double tJV = a.stab ? tauJ * V : 0.0;
+
+  // QoI value and the weight of its derivative
+  double ks_w = 0.0;
+  if (a.qoi == QOI_AVG_DISP) {
+    double ev = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      ev += (((pt.un[0][i] * 0.25 + pt.un[1][i] * 0.25) + pt.un[2][i] * 0.25) + pt.un[3][i] * 0.25) * V;
+    a.qoi_elem[s] = ev * kThird;
+  } else if (a.qoi == QOI_KS_VM) {
+    const double(&sg)[3][3] = pt.sg;
+    double d1 = sg[0][0] - sg[1][1], d2 = sg[1][1] - sg[2][2], d3 = sg[2][2] - sg[0][0];
+    double s7 = 0.5 * (d1 * d1 + d2 * d2 + d3 * d3 + 6.0 * (sg[0][1] * sg[0][1] + sg[1][2] * sg[1][2] + sg[2][0] * sg[2][0]));
+    double ex = exp(a.rho * (sqrt(s7) - a.ks_max));
+    a.qoi_elem[s] = (1.0 / (a.rho * a.ks_scale)) * ex * V;
+    ks_w = (V / a.ks_scale) * ex;
+  }
+
+  // tangent coefficients, as in k_elem
+  const double pJ = pt.pval * J, ga = gamma * alpha;
+  double yq = 0.0, yh = 0.0, yn = 0.0;
+  const bool need_n = pt.plastic || (a.qoi == QOI_KS_VM);
+  if (pt.plastic) {
+    const double A1 = 2.0 * pt.fyield * pt.kh * (pt.rcc * pt.rcc) * pt.rsmag;
+    const double A2 = 2.0 * pt.mubar * pt.k0 * pt.rcc * (pt.rsmag * pt.rsmag);
+    yq = -A1 * (2.0 * alpha / 3.0);
+    yh = A2 * (2.0 / 3.0) * pt.smag;
+    yn = -A2 * (2.0 * alpha * pt.rsmag);
+  }
+  double vq = 0.0, vh = 0.0, vn = 0.0;  // dM/du (KS): c1 (vq q + vh h + vn n)
+  if (a.qoi == QOI_KS_VM) {
+    double fs = 1.0, fmu = 0.0;
+    if (pt.plastic) { fs = pt.kh / pt.cc; fmu = -2.0 * pt.fyield * pt.kh / (pt.cc * pt.cc); }
+    const double c1 = ks_w * 1.22474487139158904909 * Jinv;  // sqrt(3/2)/J
+    vh = c1 * (fs * (-(2.0 / 3.0) * pt.smag) - gamma * pt.smag);
+    vn = c1 * (fs * (2.0 * alpha / pt.smag));
+    vq = c1 * (fmu * (2.0 * alpha / 3.0));
+  }
+  const double xm = V * (-(2.0 / 3.0) * ga), xh = V * pJ;
+  const double yhc = V * (-(2.0 / 3.0) * ga + alpha * yh), yqc = V * (alpha * yq), ync = V * (alpha * yn);
+  const double zs = V * (ga * Ic3 - pJ), gaV = ga * V;
+  const double upf = V * J * 0.25, ppc = V * pt.pp_coef, pu0 = V * ((J + Jinv) * 0.125);
+
+  // Fixed point from here on. Element scales: bL of F C and F^-T, bS of s, bX and
+  // bY of the coefficients of X, Z and of Y.
+  auto high3 = [](int l, const double(&x)[3][3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) l = max(l, fx_high(x[i][k]));
+    return l;
+  };
+  int lS = 0;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) lS = max(lS, fx_high(pt.s[q]));
+  const int lL = high3(high3(0, FC), H);
+  const int lX = max(max(fx_high(xm), fx_high(xh)), fx_high(zs)), lY = max(fx_high(yhc), fx_high(yqc));
+  int all = max(max(lL, max(lX, lY)), max(lS, max(fx_high(ync), fx_high(Ic3))));
+  const int bL = fx_exp(lL), bS = fx_exp(lS), bI = fx_exp(fx_high(Ic3));
+  const int bX = fx_exp(lX), bY = max(fx_exp(lY), need_n ? fx_exp(fx_high(ync)) + bS - 1020 : 0);
+  const int grow = max(bI - 1022, 0);
+  Fx fFC[3][3], fS[6];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) fFC[i][k] = fx_factor(FC[i][k], bL);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) fS[q] = fx_factor(pt.s[q], bS);
+  const Fx fI = fx_factor(Ic3, bI), fxm = fx_factor(xm, bX), fxh = fx_factor(xh, bX), fzs = fx_factor(zs, bX);
+  const Fx fyh = fx_factor(yhc, bY), fyq = fx_factor(yqc, bY), fyn = fx_factor(ync, bY - bS + 1020);
+
+  // Per node n, at the unit x_n = bL + bG_n + grow - 2101: h (from FP64, which R
+  // needs), m = F C G, q = m - Ic/3 h; X, Z at x_n + bX - 1023, Y at x_n + bY -
+  // 1023. Their largest sizes, packed 8 bits a node.
+  unsigned long long bGs = 0;
+  unsigned sh = 0, sq = 0, sx = 0, sy = 0;
+#pragma unroll 1
+  for (int n = 0; n < 4; ++n) {
+    double G[3], hv[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) G[k] = __ldg(a.d.grads + (3 * n + k) * E + s);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) hv[i] = H[i][0] * G[0] + H[i][1] * G[1] + H[i][2] * G[2];
+    const double w = vv[0] * hv[0] + vv[1] * hv[1] + vv[2] * hv[2];
+    double Ru[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) Ru[i] = fma(TV[i][0], hv[0], fma(TV[i][1], hv[1], TV[i][2] * hv[2]));
+    st4(rec_r + 4 * n, Ru[0], Ru[1], Ru[2], fma(tJV, w, rp0));
+    if (a.qoi == QOI_AVG_DISP) {
+      const double d = V * (1.0 / 12.0);
+      st4(a.dbuf + 16ll * (s - a.ebase) + 4 * n, d, d, d, 0.0);
+    }
+    const int lG = max(fx_high(G[0]), max(fx_high(G[1]), fx_high(G[2]))), bG = fx_exp(lG);
+    all = max(max(all, lG), max(fx_high(hv[0]), max(fx_high(hv[1]), fx_high(hv[2]))));
+    bGs |= (unsigned long long)bG << (16 * n);
+    const int xn = bL + bG + grow - 2101;
+    Fx fG[3], fm[3], fh[3], fq[3], fn[3];
+    double dM[3];  // d (KS) / du = vq q + vh h + vn n
+#pragma unroll
+    for (int k = 0; k < 3; ++k) fG[k] = fx_factor(G[k], bG);
+    unsigned long long mh = 0, mq = 0, mx = 0, my = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      FxSum m, c;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        m.add(fFC[i][k], fG[k]);
+        m.add_low(fFC[i][k], fG[k]);
+      }
+      const int down = min(4 + grow, 62);
+      const long long mi = (m.value5() + (1ll << (down - 1))) >> down, hi = fx_at(hv[i], xn);
+      fm[i] = fx_split(mi);
+      fh[i] = fx_split(hi);
+      c.add(fI, fh[i]);
+      c.add_low(fI, fh[i]);
+      const long long qi = mi - fx_scale(c.value5(), bI - 1023);
+      fq[i] = fx_split(qi);
+      if (a.qoi == QOI_KS_VM) dM[i] = vq * fx_double(qi, xn) + vh * hv[i];
+      slot[at(0, n, i) * kFixThreads] = hi;
+      slot[at(1, n, i) * kFixThreads] = qi;
+      mh |= fx_abs(hi);
+      mq |= fx_abs(qi);
+    }
+    if (need_n) {
+      FxSum n0, n1, n2;
+      n0.add(fS[0], fm[0]); n0.add(fS[3], fm[1]); n0.add(fS[5], fm[2]);
+      n1.add(fS[3], fm[0]); n1.add(fS[1], fm[1]); n1.add(fS[4], fm[2]);
+      n2.add(fS[5], fm[0]); n2.add(fS[4], fm[1]); n2.add(fS[2], fm[2]);
+      const long long nv[3] = {n0.value5() >> 3, n1.value5() >> 3, n2.value5() >> 3};
+#pragma unroll
+      for (int k = 0; k < 3; ++k) fn[k] = fx_split(nv[k]);
+      if (a.qoi == QOI_KS_VM)
+        st4(a.dbuf + 16ll * (s - a.ebase) + 4 * n, dM[0] + vn * fx_double(nv[0], xn + bS - 1020),
+            dM[1] + vn * fx_double(nv[1], xn + bS - 1020), dM[2] + vn * fx_double(nv[2], xn + bS - 1020), 0.0);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      FxSum X, Y, Z;
+      X.add(fxm, fm[k]);
+      X.add(fxh, fh[k]);
+      Y.add(fyh, fh[k]);
+      if (need_n) {
+        Y.add(fyq, fq[k]);
+        Y.add(fyn, fn[k]);
+      }
+      Z.add(fzs, fh[k]);
+      const long long x = X.value5(), y = Y.value5(), z = Z.value5();
+      slot[at(2, n, k) * kFixThreads] = x;
+      slot[at(3, n, k) * kFixThreads] = y;
+      slot[at(4, n, k) * kFixThreads] = z;
+      mx |= fx_abs(x) | fx_abs(z);
+      my |= fx_abs(y);
+    }
+    sh |= (unsigned)fx_bits(mh) << (8 * n);
+    sq |= (unsigned)fx_bits(mq) << (8 * n);
+    sx |= (unsigned)fx_bits(mx) << (8 * n);
+    sy |= (unsigned)fx_bits(my) << (8 * n);
+  }
+
+  // The final scales. h_n: shifted to 62 bits, unit xl_n. X_n, Z_n: unit xl_n +
+  // F. q_n is far smaller than h_n near the undeformed state and a plastic Y_n
+  // far larger than X_n, so they have their own: q_n unit xl_n - up, Y_n unit
+  // xl_n + FY; their products come `down` bits finer than the others.
+  auto byte_of = [](unsigned x, int n) { return (int)((x >> (8 * n)) & 255u); };
+  auto bG_of = [&](int n) { return (int)(bGs >> (16 * n)) & 0xffff; };
+  auto xl_of = [&](int n) { return bL + bG_of(n) + grow - 2163 + byte_of(sh, n); };
+  int F = -32768, FY = -32768, up = 32767;
+#pragma unroll 1
+  for (int n = 0; n < 4; ++n) {
+    const int h0 = 1022 + byte_of(sh, n);
+    F = max(F, bX - h0 - 1 + byte_of(sx, n));
+    FY = max(FY, bY - h0 - 1 + byte_of(sy, n));
+    up = min(up, byte_of(sh, n) - byte_of(sq, n));
+  }
+  F = max(F, FY - up);
+  // c_ab = ga V G_a . C G_b of the pairs (in FP64: two numbers to quantize for
+  // each would cost more)
+#pragma unroll 1
+  for (int n = 0, p = 0; n < 3; ++n) {
+    double G[3], CG[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) G[k] = __ldg(a.d.grads + (3 * n + k) * E + s);
+    if constexpr (MODEL == MODEL_J2) {
+      CG[0] = gaV * (pt.C[0] * G[0] + pt.C[3] * G[1] + pt.C[5] * G[2]);
+      CG[1] = gaV * (pt.C[3] * G[0] + pt.C[1] * G[1] + pt.C[4] * G[2]);
+      CG[2] = gaV * (pt.C[5] * G[0] + pt.C[4] * G[1] + pt.C[2] * G[2]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) CG[k] = gaV * G[k];
+    }
+#pragma unroll 1
+    for (int b = n + 1; b < 4; ++b, ++p) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) G[k] = __ldg(a.d.grads + (3 * b + k) * E + s);
+      const double c = fma(CG[0], G[0], fma(CG[1], G[1], CG[2] * G[2]));
+      all = max(all, fx_high(c));
+      F = max(F, fx_exp(fx_high(c)) - 1146 - xl_of(n) - xl_of(b));
+      slot[(kFixC + p) * kFixThreads] = __double_as_longlong(c);
+    }
+  }
+
+  // scales of the other entries, and the factors
+  double tvv[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) tvv[k] = tJV * vv[k];
+  const int lt = max(fx_high(tvv[0]), max(fx_high(tvv[1]), fx_high(tvv[2])));
+  const int bT = fx_exp(lt), bJ = fx_exp(fx_high(tJV)), bU = fx_exp(fx_high(upf));
+  const int bP = fx_exp(fx_high(pu0)), xc = fx_exp(fx_high(ppc)) - 1082;
+  all = max(max(all, lt), max(max(fx_high(tJV), fx_high(upf)), max(fx_high(pu0), fx_high(ppc))));
+  const bool bad = all >= 0x7ff00000;
+  const Fx fJ = fx_factor62(tJV, bJ), fU = fx_factor62(upf, bU), fP = fx_factor62(pu0, bP);
+  const long long mass = fx_at(ppc, xc);
+  Fx ft[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) ft[k] = fx_factor62(tvv[k], bT);
+  const int down = F + up - FY;
+  // h_n is in units 2^(exp_of(n) - 1082)
+  auto exp_of = [&](int n) { return xl_of(n) + 1082; };
+#pragma unroll 1
+  for (int n = 0; n < 4; ++n) {
+    const int dh = 62 - byte_of(sh, n), dx = dh + bX - 1023 - F, dy = dh + bY - 1023 - FY;
+    long long w = 0;  // tau J V v . h_n
+#pragma unroll
+    for (int q = 0; q < 15; ++q) {
+      const int i = at(q / 3, n, q % 3);
+      const Fx f = fx_split(fx_scale(slot[i * kFixThreads], q < 3 ? dh : q < 6 ? dh + up : q >= 9 && q < 12 ? dy : dx));
+      put_factor(i, f);
+      if (q < 3) w += fx_mul(ft[q], f);
+    }
+    put_factor(kFixW + n, fx_split(w));
+  }
+
+  auto store_row = [&](long long* p, long long x0, long long x1, long long x2, long long x3) {
+    st4(reinterpret_cast<double*>(p), __longlong_as_double(x0), __longlong_as_double(x1), __longlong_as_double(x2),
+        __longlong_as_double(x3));
+  };
+  auto store_exps = [&](int r, int c, int uu, int up, int pu, int pp) {
+    reinterpret_cast<short4*>(rec + kRecExp)[4 * r + c] =
+        bad ? make_short4(kFxBad, kFxBad, kFxBad, kFxBad) : make_short4((short)uu, (short)up, (short)pu, (short)pp);
+  };
+  // e_ab = h_a . h_b, and K^pp: the pressure mass term and tau J e_ab at a common scale
+  auto pp_block = [&](const Fx& e, int er, int ec, int& x) {
+    const int xj = bJ + er + ec - 3120;
+    long long r = mass;
+    fx_acc(r, xc, fx_mul(e, fJ), xj);
+    x = max(xc, xj);
+    return r;
+  };
+#pragma unroll 1
+  for (int r = 0, p = 0; r < 4; ++r) {
+    const int er = exp_of(r);
+    Fx hr[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) hr[k] = factor(at(0, r, k));
+    {  // column 3 of the diagonal block
+      const Fx e = fx_split(fx_mul(hr[0], hr[0]) + fx_mul(hr[1], hr[1]) + fx_mul(hr[2], hr[2]));
+      int xpp;
+      const long long pp = pp_block(e, er, er, xpp);
+      store_row(rec + kRecDiag + 4 * r, fx_mul(fU, hr[0]), fx_mul(fU, hr[1]), fx_mul(fU, hr[2]), pp);
+      store_exps(r, r, kFxBad, bU + er - 2102, kFxBad, xpp);
+    }
+#pragma unroll 1
+    for (int c = r + 1; c < 4; ++c, ++p) {
+      const int ec = exp_of(c);
+      const int x = er + ec + F - 2100;
+      const long long cab =
+          fx_at(__longlong_as_double(slot[(kFixC + p) * kFixThreads]), x);
+      Fx hc[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) hc[k] = factor(at(0, c, k));
+      long long P[3][3];  // h_c Z_r + c_ab I: shared by the pair
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const Fx z = factor(at(4, r, k));
+#pragma unroll
+        for (int i = 0; i < 3; ++i) P[i][k] = fx_mul(hc[i], z) + (i == k ? cab : 0);
+      }
+      const Fx e = fx_split(fx_mul(hr[0], hc[0]) + fx_mul(hr[1], hc[1]) + fx_mul(hr[2], hc[2]));
+      const Fx wr = factor(kFixW + r), wc = factor(kFixW + c);
+      int xpp;
+      const long long pp = pp_block(e, er, ec, xpp);
+      // K^pu, stabilization: w_r h_c - w_c h_r - e v at xs, and the term with the other node's h
+      const int xs = bT + er + ec - 3120;
+      long long D[3], T3[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        D[k] = fx_mul(wr, hc[k]) - fx_mul(wc, hr[k]);
+        T3[k] = fx_mul(e, ft[k]);
+      }
+      auto block = [&](int row, int col, const Fx(&hrow)[3], const Fx(&hcol)[3], int erow, int ecol, bool flip) {
+        long long* blk = rec + kRecOff + 16 * off_index(row, col);
+        Fx X[3], Y[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          X[k] = factor(at(2, col, k));
+          Y[k] = factor(at(3, col, k));
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const Fx q = factor(at(1, row, i));
+          long long K[3];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            K[k] = fx_mul(hrow[i], X[k]) + (fx_mul(q, Y[k]) >> min(down, 63)) + (flip ? P[k][i] : P[i][k]);
+          }
+          store_row(blk + 4 * i, K[0], K[1], K[2], fx_mul(fU, hrow[i]));
+        }
+        const int xp = bP + ecol - 2102;
+        long long K3[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          K3[k] = -fx_mul(fP, hcol[k]);
+          fx_acc(K3[k], xp, (flip ? -D[k] : D[k]) - T3[k], xs);
+        }
+        store_row(blk + 12, K3[0], K3[1], K3[2], pp);
+        store_exps(row, col, x, bU + erow - 2102, max(xp, xs), xpp);
+      };
+      block(r, c, hr, hc, er, ec, false);
+      block(c, r, hc, hr, ec, er, true);
+    }
+  }
 }
 
 // ------------------------------------------------------------------ reductions
@@ -687,19 +1137,12 @@ __global__ void k_fill_identity(int E, double* Fp) {
 }
 
 template <int MODEL, int MODE, bool JAC, bool ERR>
-void launch_colours(const Disc& d, ElemArgs args, cudaStream_t st, bool buffered, bool dsum = false) {
+void launch_colours(const Disc& d, ElemArgs args, cudaStream_t st, bool buffered) {
   const int block = 128;
   if (MODE == MODE_NONE || buffered) {
     // elements [args.begin, args.end) into the buffer (all of them, or a chunk)
     const int n = args.end - args.begin;
     if (n <= 0) return;
-    if constexpr (JAC && MODE != MODE_NONE) {
-      if (dsum) {
-        k_elem<MODEL, MODE, JAC, ERR, true, true><<<(n + block - 1) / block, block, 0, st>>>(args);
-        GOAL_CHECK_LAUNCH();
-        return;
-      }
-    }
     k_elem<MODEL, MODE, JAC, ERR, true><<<(n + block - 1) / block, block, 0, st>>>(args);
     GOAL_CHECK_LAUNCH();
   } else {
@@ -715,21 +1158,28 @@ void launch_colours(const Disc& d, ElemArgs args, cudaStream_t st, bool buffered
 }
 
 template <int MODEL>
-void dispatch(const Disc& d, const Chain& c, const ElemArgs& args, cudaStream_t st, bool buf, bool dsum) {
+void dispatch(const Disc& d, const Chain& c, const ElemArgs& args, cudaStream_t st, bool buf, bool fix) {
   if (c.error_chain) {
     GOAL_REQUIRE(!c.jacobian && c.mode == MODE_PRIMAL, GOAL_ERR_ARG, "the error chain is a residual (PRIMAL) chain");
     launch_colours<MODEL, MODE_PRIMAL, false, true>(d, args, st, buf);
+    return;
+  }
+  if (fix) {
+    constexpr int smem = kFixSlots * kFixThreads * (int)sizeof(long long);
+    GOAL_CUDA(cudaFuncSetAttribute(k_elem_fix<MODEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_elem_fix<MODEL><<<(args.end - args.begin + kFixThreads - 1) / kFixThreads, kFixThreads, smem, st>>>(args);
+    GOAL_CHECK_LAUNCH();
     return;
   }
   if (c.mode == MODE_NONE) {
     if (c.jacobian) launch_colours<MODEL, MODE_NONE, true, false>(d, args, st, true);
     else launch_colours<MODEL, MODE_NONE, false, false>(d, args, st, true);
   } else if (c.mode == MODE_PRIMAL) {
-    if (c.jacobian) launch_colours<MODEL, MODE_PRIMAL, true, false>(d, args, st, buf, dsum);
+    if (c.jacobian) launch_colours<MODEL, MODE_PRIMAL, true, false>(d, args, st, buf);
     else launch_colours<MODEL, MODE_PRIMAL, false, false>(d, args, st, buf);
   } else {
     GOAL_REQUIRE(c.jacobian, GOAL_ERR_ARG, "ADJOINT mode is a Jacobian (FADT) chain");
-    launch_colours<MODEL, MODE_ADJOINT, true, false>(d, args, st, buf, dsum);
+    launch_colours<MODEL, MODE_ADJOINT, true, false>(d, args, st, buf);
   }
 }
 
@@ -814,52 +1264,6 @@ __global__ void __launch_bounds__(256) k_gather_blocks_chunk(int count, const in
   }
 }
 
-// Phase 2 for the diagonal blocks after a DSUM element phase, once the
-// off-diagonal blocks are gathered: thread (node n, row r). PRIMAL: the u
-// columns of row r are the negated sum of row r of the row's off-diagonal
-// blocks; column 3 sums the elements' packed column-3 contributions in element
-// order. TRANSPOSE (ADJOINT mode stores dR/du^T): rows 0..2 are the negated
-// sums of the same rows of the blocks (m, n) of the block column (btr), row 3
-// sums the packed contributions. No atomics; fixed order.
-template <bool TRANSPOSE>
-__global__ void __launch_bounds__(256) k_gather_diag(int N, const int* __restrict__ brow_ptr,
-                                                     const int* __restrict__ diag, const int* __restrict__ btr,
-                                                     const int* __restrict__ bptr, const int* __restrict__ blist,
-                                                     const double* __restrict__ ebuf, int estride,
-                                                     double* __restrict__ A) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < 4ll * N;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int n = (int)(t >> 2), r = (int)(t & 3);
-    const int kd = __ldg(diag + n), k0 = __ldg(brow_ptr + n), k1 = __ldg(brow_ptr + n + 1);
-    const int c0 = __ldg(bptr + kd), c1 = __ldg(bptr + kd + 1);
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    if (!TRANSPOSE || r < 3) {
-      for (int k = k0; k < k1; ++k) {
-        if (k == kd) continue;
-        const int kk = TRANSPOSE ? __ldg(btr + k) : k;
-        double x0, x1, x2, x3;
-        ld4(A + 16ll * kk + 4 * r, x0, x1, x2, x3);
-        a0 -= x0; a1 -= x1; a2 -= x2;
-        if (TRANSPOSE) a3 -= x3;
-      }
-    }
-    if (!TRANSPOSE) {
-      for (int c = c0; c < c1; ++c) {
-        const int v = __ldg(blist + c);
-        a3 += __ldg(ebuf + (size_t)(v >> 4) * estride + 16 + 16 * (v & 15) + r);
-      }
-    } else if (r == 3) {
-      for (int c = c0; c < c1; ++c) {
-        const int v = __ldg(blist + c);
-        double x0, x1, x2, x3;
-        ld4(ebuf + (size_t)(v >> 4) * estride + 16 + 16 * (v & 15), x0, x1, x2, x3);
-        a0 += x0; a1 += x1; a2 += x2; a3 += x3;
-      }
-    }
-    st4(A + 16ll * kd + 4 * r, a0, a1, a2, a3);
-  }
-}
-
 // Phase 2 for nodal vectors: node n, row q sums the element rows of its
 // incident elements (entries 4*s + a of nlist) in element order.
 // [lo, hi): the element slots the buffer holds (a chunk; the buffer's first
@@ -879,6 +1283,238 @@ __global__ void __launch_bounds__(256) k_gather_nodes(int N, const int* __restri
       acc += __ldg(ebuf + (size_t)(e - lo) * estride + 4 * (v & 3) + q);
     }
     out[t] = acc;
+  }
+}
+
+// One lane's share of a diagonal block's row: the sum of the row's
+// off-diagonal blocks, 96 bits at a common exponent.
+struct RowSum {
+  long long h[3] = {0, 0, 0}, l[3] = {0, 0, 0};  // h 2^32 + l
+  int x = -32768;
+  __device__ __forceinline__ void raise(int to) {  // to the larger exponent `to`
+    const int d = min(to - x, 95);
+    if (d > 0) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const long long hh = h[k] + (l[k] >> 32);
+        const unsigned ll = (unsigned)l[k];
+        const unsigned h0 = (unsigned)hh;
+        l[k] = d < 32 ? (unsigned)((((unsigned long long)h0 << 32) | ll) >> d) : (unsigned)(hh >> min(d - 32, 63));
+        h[k] = hh >> min(d, 63);
+      }
+    }
+    x = max(x, to);
+  }
+  __device__ __forceinline__ void add(const long long (&v)[4], int xv) {
+    raise(xv);
+    const int d = fx_shift(x - xv);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const long long s = v[k] >> d;
+      h[k] += s >> 32;
+      l[k] += (unsigned)s;
+    }
+  }
+};
+
+// Phase 2 after a FIX element phase. The first row_blocks blocks of the grid
+// take one matrix block row to a warp: a quad of lanes sums the contributions
+// of one off-diagonal block (a lane per row of it) in integers aligned to the
+// largest exponent met, and the warp then forms the diagonal block: its u
+// columns as the negated sum of the row's off-diagonal blocks, column 3 from
+// the elements' diagonal records. ADJ stores the transpose (dR/du^T): block
+// (n, m) goes to block (m, n). The remaining blocks sum the nodal vectors, as
+// k_gather_nodes does (four threads per node, element order): R from the
+// records, and dM/du from dbuf if there is one.
+// The sums need no FP64 instruction but one conversion per matrix entry. At
+// 384,000 elements 231 us (3.9 TB/s; latency and the integer pipes, 47% busy)
+// against 268 us for the FP64 gathers, which the shorter element phase and the
+// single launch come on top of; with the lists fetched where they are used the
+// kernel took 257 us, with the lists of two passes in registers 283 us.
+constexpr int kRowTerms = 192;  // list entries of a row kept in shared memory (96 on the Kuhn grid)
+template <bool ADJ>
+__global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, const int* __restrict__ brow_ptr,
+                                                     const int* __restrict__ diag, const int* __restrict__ btr,
+                                                     const int* __restrict__ bptr, const int* __restrict__ blist,
+                                                     const int* __restrict__ nptr, const int* __restrict__ nlist,
+                                                     const long long* __restrict__ rec, double* __restrict__ A,
+                                                     double* __restrict__ R, const double* __restrict__ dbuf,
+                                                     double* __restrict__ dMdu) {
+  if ((int)blockIdx.x >= row_blocks) {
+    const long long vectors = dbuf ? 2 : 1;
+    for (long long t = (blockIdx.x - row_blocks) * (long long)blockDim.x + threadIdx.x; t < vectors * 4ll * N;
+         t += (long long)(gridDim.x - row_blocks) * blockDim.x) {
+      const bool second = t >= 4ll * N;
+      const long long i = second ? t - 4ll * N : t;
+      const int n = (int)(i >> 2), q = (int)(i & 3);
+      const double* src = second ? dbuf : reinterpret_cast<const double*>(rec);
+      const int stride = second ? 16 : kRecord;
+      double acc = 0.0;
+      const int c1 = __ldg(nptr + n + 1);
+#pragma unroll 4
+      for (int c = __ldg(nptr + n); c < c1; ++c) {
+        const int v = __ldg(nlist + c);
+        acc += __ldg(src + (size_t)(v >> 2) * stride + 4 * (v & 3) + q);
+      }
+      (second ? dMdu : R)[i] = acc;
+    }
+    return;
+  }
+  const int lane = threadIdx.x & 31, q = lane >> 2, r = lane & 3;
+  const unsigned full = 0xffffffffu;
+  // the 4x4 block whose row r a lane of the quad holds, transposed
+  auto transpose = [&](double (&d)[4]) {
+    const bool hi = (r & 2) != 0, odd = (r & 1) != 0;
+    const double s0 = __shfl_xor_sync(full, hi ? d[0] : d[2], 2), s1 = __shfl_xor_sync(full, hi ? d[1] : d[3], 2);
+    const double a0 = hi ? s0 : d[0], a1 = hi ? s1 : d[1], a2 = hi ? d[2] : s0, a3 = hi ? d[3] : s1;
+    const double t0 = __shfl_xor_sync(full, odd ? a0 : a1, 1), t1 = __shfl_xor_sync(full, odd ? a2 : a3, 1);
+    d[0] = odd ? t0 : a0; d[1] = odd ? a1 : t0; d[2] = odd ? t1 : a2; d[3] = odd ? a3 : t1;
+  };
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  constexpr int kNone = -32768;  // exponent of no term: every shift takes it to zero
+  __shared__ int lists[4][kRowTerms];
+  int* mine = lists[threadIdx.x >> 5];
+  // T terms of a block from list entries w (those past `left` are none): the
+  // accumulators go to the largest exponent once, then every term is added there
+  auto add = [&](auto count, const int* w, int left, int extra, long long (&acc)[4], int& x0, int& x3) {
+    constexpr int T = decltype(count)::value;
+    int e0[T], e3[T], m0 = x0, m3 = x3;
+    longlong4_32a v[T];
+#pragma unroll
+    for (int u = 0; u < T; ++u) {
+      e0[u] = e3[u] = kNone;
+      v[u] = longlong4_32a{0, 0, 0, 0};
+      if (u < left) {
+        const int l = w[u];
+        const long long* p = rec + (size_t)(l >> 4) * kRecord;
+        const int e = __ldg(reinterpret_cast<const int*>(p + kRecExp + (l & 15)) + (r == 3 ? 1 : 0));
+        v[u] = *reinterpret_cast<const longlong4_32a*>(p + kRecOff + 16 * off_index((l >> 2) & 3, l & 3) + 4 * r);
+        e0[u] = (short)e + extra;
+        e3[u] = (e >> 16) + extra;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < T; ++u) {
+      m0 = max(m0, e0[u]);
+      m3 = max(m3, e3[u]);
+    }
+    if (m0 > x0) {
+      const int s0 = min(m0 - x0, 62);
+      const long long h0 = (1ll << s0) >> 1;
+      acc[0] = (acc[0] + h0) >> s0; acc[1] = (acc[1] + h0) >> s0; acc[2] = (acc[2] + h0) >> s0;
+    }
+    if (m3 > x3) {
+      const int s3 = min(m3 - x3, 62);
+      acc[3] = (acc[3] + ((1ll << s3) >> 1)) >> s3;
+    }
+#pragma unroll
+    for (int u = 0; u < T; ++u) {
+      const int d0 = min(m0 - e0[u] + extra, 62), d3 = min(m3 - e3[u] + extra, 62);
+      const long long h0 = (1ll << d0) >> 1, h3 = (1ll << d3) >> 1;  // to round
+      acc[0] += (v[u].x + h0) >> d0; acc[1] += (v[u].y + h0) >> d0; acc[2] += (v[u].z + h0) >> d0;
+      acc[3] += (v[u].w + h3) >> d3;
+    }
+    x0 = m0;
+    x3 = m3;
+  };
+  for (int n = blockIdx.x * 4 + (threadIdx.x >> 5); n < N; n += row_blocks * 4) {
+    // the lists of the whole row before any record: its block pointers (one a
+    // lane) and its terms (in shared memory) are contiguous
+    const int k0 = __ldg(brow_ptr + n), nk = __ldg(brow_ptr + n + 1) - k0, nb = nk - 1, kd = __ldg(diag + n) - k0;
+    const int bp = __ldg(bptr + k0 + min(lane, nk));
+    const int t0 = __shfl_sync(full, bp, 0), t1 = nk < 32 ? __shfl_sync(full, bp, nk) : __ldg(bptr + k0 + nk);
+    const bool ahead = t1 - t0 <= kRowTerms;
+    const int* terms = ahead ? mine - t0 : blist;  // list entry c is terms[c]
+    __syncwarp();
+    if (ahead)
+      for (int i = lane; i < t1 - t0; i += 32) mine[i] = __ldg(blist + t0 + i);
+    __syncwarp();
+    auto range = [&](int k, int& c0, int& c1) {  // of block k of the row; all lanes call it
+      c0 = __shfl_sync(full, bp, k & 31);
+      c1 = __shfl_sync(full, bp, (k + 1) & 31);
+      if (k >= 31 && k < nk) {
+        c0 = __ldg(bptr + k0 + k);
+        c1 = __ldg(bptr + k0 + k + 1);
+      }
+    };
+    RowSum row;
+    for (int i0 = 0; i0 < nb; i0 += 8) {
+      const bool live = i0 + q < nb;
+      const int k = i0 + q + (i0 + q >= kd ? 1 : 0);
+      int c, c1;
+      range(k, c, c1);
+      double d[4] = {0.0, 0.0, 0.0, 0.0};
+      if (live) {
+        const int extra = c1 - c > 1 ? 32 - __clz(c1 - c - 1) : 0;  // room for that many terms below 2^62
+        long long acc[4] = {0, 0, 0, 0};
+        int x0 = kNone, x3 = kNone;
+        for (; c < c1; c += 4) {
+          if (c1 - c > 2) add(std::integral_constant<int, 4>(), terms + c, c1 - c, extra, acc, x0, x3);
+          else add(std::integral_constant<int, 2>(), terms + c, c1 - c, extra, acc, x0, x3);
+        }
+        row.add(acc, x0);
+        const bool bad0 = x0 >= kFxBad, bad3 = x3 >= kFxBad;
+        d[0] = bad0 ? nan : fx_double(acc[0], x0);
+        d[1] = bad0 ? nan : fx_double(acc[1], x0);
+        d[2] = bad0 ? nan : fx_double(acc[2], x0);
+        d[3] = bad3 ? nan : fx_double(acc[3], x3);
+      }
+      if (ADJ) transpose(d);
+      if (live) st4(A + 16ll * (ADJ ? __ldg(btr + k0 + k) : k0 + k) + 4 * r, d[0], d[1], d[2], d[3]);
+    }
+    // column 3 of the diagonal block: the terms of block kd are the node's elements
+    long long dacc = 0;
+    int dx = kNone;
+    {
+      int c, c1;
+      range(kd, c, c1);
+      const int extra = c1 - c > 2 ? 31 - __clz(c1 - c - 1) : 0;  // terms below 2^61
+#pragma unroll 2
+      for (int i = c + q; i < c1; i += 8) {
+        const int l = terms[i];
+        const long long* p = rec + (size_t)(l >> 4) * kRecord;
+        const int e = (__ldg(reinterpret_cast<const int*>(p + kRecExp + (l & 15)) + (r == 3 ? 1 : 0)) >> 16) + extra;
+        const int top = max(dx, e), sa = min(top - dx, 62), sv = min(top - e + extra, 62);
+        const long long v = __ldg(p + kRecDiag + 4 * (l & 3) + r);
+        dacc = ((dacc + ((1ll << sa) >> 1)) >> sa) + ((v + ((1ll << sv) >> 1)) >> sv);
+        dx = top;
+      }
+    }
+    // sums over the quads: exponents first, then the integers
+    int rx = row.x, ex = dx;
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      rx = max(rx, __shfl_xor_sync(full, rx, o));
+      ex = max(ex, __shfl_xor_sync(full, ex, o));
+    }
+    dacc >>= fx_shift(ex - dx);
+    row.raise(rx);
+    // the row sums as 64 bits, shifted so far that eight of them cannot overflow
+    long long t[3];
+    int bits = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      t[k] = row.h[k] + (row.l[k] >> 32);
+      bits = max(bits, 64 - __clzll(t[k] ^ (t[k] >> 63)));
+    }
+    bits = __reduce_max_sync(full, bits);
+    const int sh = min(max(bits - 27, 0), 32);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      t[k] = sh == 32 ? t[k] : (t[k] << (32 - sh)) | (long long)((unsigned)row.l[k] >> sh);
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      dacc += __shfl_xor_sync(full, dacc, o);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) t[k] += __shfl_xor_sync(full, t[k], o);
+    }
+    double d[4];
+    const bool badr = rx >= kFxBad, badd = ex >= kFxBad;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) d[k] = badr ? nan : fx_double(-t[k], rx + sh);
+    d[3] = badd ? nan : fx_double(dacc, ex);
+    if (ADJ) transpose(d);
+    if (q == 0) st4(A + 16ll * (k0 + kd) + 4 * r, d[0], d[1], d[2], d[3]);
   }
 }
 
@@ -1089,10 +1725,17 @@ double assemble(Mechanics& m, SolInfo* s, const Chain& c, const ErrorWeights* w,
   const bool scatter = c.mode != MODE_NONE;
   const int E = d.num_elems;
   int chunk = E;  // elements per pass of the two-phase assembly
+  bool fix = false;
   if (buf) {
     a.estride = c.jacobian ? 272 : 16;
     const size_t per_elem = sizeof(double) * (a.estride + ((c.jacobian && c.qoi != QOI_NONE) ? 16 : 0));
     chunk = (int)std::max<long long>(1, std::min<long long>(E, element_buffer_limit() / per_elem));
+    // fixed point and diagonal blocks from row sums: Jacobian chains that overwrite, in one pass
+    fix = scatter && c.jacobian && c.overwrite && chunk == E;
+    if (fix) {
+      a.estride = kRecord;
+      if (c.mode == MODE_ADJOINT) const_cast<Disc&>(d).block_transpose_map();
+    }
     size_t need = (size_t)chunk * a.estride;
     if (m.ebuf.n < need) m.ebuf.alloc(need);
     a.ebuf = m.ebuf.ptr;
@@ -1101,9 +1744,6 @@ double assemble(Mechanics& m, SolInfo* s, const Chain& c, const ErrorWeights* w,
       a.dbuf = m.dbuf.ptr;
     }
   }
-  // diagonal blocks from row sums: buffered Jacobian chains that overwrite, in one pass
-  const bool dsum = buf && scatter && c.jacobian && c.overwrite && chunk == E;
-  if (dsum && c.mode == MODE_ADJOINT) const_cast<Disc&>(d).block_transpose_map();
   const bool timed = g_phase.on;
   if (timed) GOAL_CUDA(cudaEventRecord(g_phase.ev[0], st));
   for (int e0 = 0; e0 < E; e0 += chunk) {
@@ -1111,10 +1751,22 @@ double assemble(Mechanics& m, SolInfo* s, const Chain& c, const ErrorWeights* w,
     a.begin = e0;
     a.end = e1;
     a.ebase = e0;
-    if (m.model == MODEL_J2) dispatch<MODEL_J2>(d, c, a, st, buf, dsum);
-    else dispatch<MODEL_NEOHOOKEAN>(d, c, a, st, buf, dsum);
+    if (m.model == MODEL_J2) dispatch<MODEL_J2>(d, c, a, st, buf, fix);
+    else dispatch<MODEL_NEOHOOKEAN>(d, c, a, st, buf, fix);
     if (timed && e0 == 0) GOAL_CUDA(cudaEventRecord(g_phase.ev[1], st));
     if (!buf) break;  // the coloured path covers every element itself
+    if (fix) {
+      const int rows = grid_for(d.num_nodes, 4, kSMs * 64);
+      const bool dm = c.qoi != QOI_NONE;
+      const int nodes = grid_for((dm ? 8ll : 4ll) * d.num_nodes, 128, kSMs * 32);
+      auto gather = c.mode == MODE_ADJOINT ? k_gather_rows<true> : k_gather_rows<false>;
+      gather<<<rows + nodes, 128, 0, st>>>(d.num_nodes, rows, d.brow_ptr.ptr, d.diag.ptr, d.btr.ptr, d.bptr.ptr,
+                                           d.blist.ptr, d.nptr.ptr, d.nlist.ptr,
+                                           reinterpret_cast<const long long*>(m.ebuf.ptr), s->A.ptr, s->R.ptr,
+                                           dm ? m.dbuf.ptr : nullptr, s->dMdu.ptr);
+      GOAL_CHECK_LAUNCH();
+      break;
+    }
     const int acc = (c.overwrite && e0 == 0) ? 0 : 1;
     const bool chunked = chunk < E;
     if (scatter) {
@@ -1128,16 +1780,7 @@ double assemble(Mechanics& m, SolInfo* s, const Chain& c, const ErrorWeights* w,
         for (int q = 0; q < 2; ++q) {
           if (counts[q] <= 0) continue;
           const int g = grid_for(4ll * counts[q], 256);
-          if (q == 1 && dsum) {  // the diagonal blocks, after the off-diagonal ones
-            if (c.mode == MODE_ADJOINT)
-              k_gather_diag<true><<<grid_for(4ll * d.num_nodes, 256), 256, 0, st>>>(
-                  d.num_nodes, d.brow_ptr.ptr, d.diag.ptr, d.btr.ptr, d.bptr.ptr, d.blist.ptr, m.ebuf.ptr,
-                  a.estride, s->A.ptr);
-            else
-              k_gather_diag<false><<<grid_for(4ll * d.num_nodes, 256), 256, 0, st>>>(
-                  d.num_nodes, d.brow_ptr.ptr, d.diag.ptr, nullptr, d.bptr.ptr, d.blist.ptr, m.ebuf.ptr,
-                  a.estride, s->A.ptr);
-          } else if (chunked) {
+          if (chunked) {
             if (c.mode == MODE_ADJOINT)
               k_gather_blocks_chunk<true><<<g, 256, 0, st>>>(counts[q], lists[q], d.bptr.ptr, d.blist.ptr, m.ebuf.ptr,
                                                              a.estride, s->A.ptr, acc, e0, e1);

@@ -45,7 +45,7 @@ struct Mechanics {
   DevBuf<double> U;         // 4N nodal solution: u_x u_y u_z p per node (the DOF layout)
   StatesDev st;
   DevBuf<double> qoi_elem;  // E   per-element QoI values (colour order)
-  DevBuf<double> ebuf;      // two-phase assembly: per-element R and 16 4x4 blocks (272 doubles)
+  DevBuf<double> ebuf;      // two-phase assembly: per-element R and blocks (fixed-point records of 240 words, or 272 doubles)
   DevBuf<double> dbuf;      // two-phase assembly: per-element dM/du (16 doubles)
   DevBuf<double> red;       // reduction scratch
   DevBuf<int> status;       // 1: return-map failures, non-finite etc.
