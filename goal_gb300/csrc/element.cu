@@ -65,7 +65,7 @@ struct ElemArgs {
   double* qoi_elem;
   const double* Zd;
   const double* Zc;
-  int* status;
+  int* failed;     // host memory: set when a return map fails
   double* ebuf;    // two-phase mode: per element [R (16) | 16 blocks x 16] (stride estride)
   double* dbuf;    // two-phase mode: per element dM/du (16)
   int estride;
@@ -262,7 +262,7 @@ __device__ __forceinline__ void eval_point(const ElemArgs& a, int s, const int (
         Xr = X1;
       }
       gamma = 1.0 - 2.0 * mubar * Xr * rsmag;
-      if (!(Xr >= 0.0) || !isfinite(Xr)) atomicOr(a.status, 1);
+      if (!(Xr >= 0.0) || !isfinite(Xr)) *a.failed = 1;
       if (a.save) {
         a.eqps[s] = eq_old + sq23 * Xr;
         // Fp = exp(dgam N) Fp_old (stored only at plastic points): the
@@ -1040,22 +1040,41 @@ __global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
 }
 
 // ------------------------------------------------------------------ reductions
-__global__ void k_sum_partial(const double* x, int n, double* part) {
-  KSum acc;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) acc.add(x[i]);
+// True in all threads of the block that finishes last; part is then complete.
+// The ticket is zero again for the next reduction.
+__device__ __forceinline__ bool last_block(unsigned* ticket) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (last) {
+      *ticket = 0u;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  return last;
+}
+__device__ __forceinline__ void put_sum(KSum acc, double* part, unsigned* ticket, double* out) {
   acc = block_reduce(acc);
   if (threadIdx.x == 0) { part[2 * blockIdx.x] = acc.s; part[2 * blockIdx.x + 1] = acc.c; }
-}
-__global__ void k_sum_final(const double* part, int nb, double* out) {
-  KSum acc;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) {
+  if (!last_block(ticket)) return;
+  KSum all;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
     KSum t;
-    t.s = part[2 * i];
-    t.c = part[2 * i + 1];
-    acc.add(t);
+    t.s = __ldcg(part + 2 * i);
+    t.c = __ldcg(part + 2 * i + 1);
+    all.add(t);
   }
-  acc = block_reduce(acc);
-  if (threadIdx.x == 0) out[0] = acc.value();
+  all = block_reduce(all);
+  if (threadIdx.x == 0) *out = all.value();
+}
+
+// The sum of x, to host memory.
+__global__ void k_sum(const double* x, int n, double* part, unsigned* ticket, double* out) {
+  KSum acc;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) acc.add(x[i]);
+  put_sum(acc, part, ticket, out);
 }
 
 __device__ __forceinline__ double vm_of(const double* sig, int E, int s) {
@@ -1065,22 +1084,30 @@ __device__ __forceinline__ double vm_of(const double* sig, int E, int s) {
   return sqrt(0.5 * (d1 * d1 + d2 * d2 + d3 * d3 + 6.0 * (a01 * a01 + a12 * a12 + a20 * a20)));
 }
 
-__global__ void k_vm_max_partial(const double* sig, int E, double* part) {
+// The largest stored von Mises stress, to device memory (for the sum) and to
+// host memory.
+__global__ void k_vm_max(const double* sig, int E, double* part, unsigned* ticket, double* out, double* host) {
   double m = 0.0;
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < E; s += gridDim.x * blockDim.x) m = fmax(m, vm_of(sig, E, s));
   m = block_max(m);
   if (threadIdx.x == 0) part[blockIdx.x] = m;
-}
-__global__ void k_max_final(const double* part, int nb, double* out) {
-  double m = 0.0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) m = fmax(m, part[i]);
+  if (!last_block(ticket)) return;
+  m = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) m = fmax(m, __ldcg(part + i));
   m = block_max(m);
-  if (threadIdx.x == 0) out[0] = m;
+  if (threadIdx.x == 0) {
+    *out = m;
+    *host = m;
+  }
 }
-__global__ void k_ks_terms(const double* sig, const double* vol, int E, double rho, const double* mx, double* out) {
-  double m = mx[0];
+// sum of exp(rho (vm - max vm)) w dv, to host memory
+__global__ void k_ks_sum(const double* sig, const double* vol, int E, double rho, const double* mx, double* part,
+                         unsigned* ticket, double* host) {
+  const double m = *mx;
+  KSum acc;
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < E; s += gridDim.x * blockDim.x)
-    out[s] = exp(rho * (vm_of(sig, E, s) - m)) * vol[s];
+    acc.add(exp(rho * (vm_of(sig, E, s) - m)) * vol[s]);
+  put_sum(acc, part, ticket, host);
 }
 
 __global__ void k_cpinv(int E, const double* Fp_old, double* Cpinv) {
@@ -1113,16 +1140,16 @@ __global__ void k_cpinv(int E, const double* Fp_old, double* Cpinv) {
 }
 
 // Fp = exp(A) Fp_old at points with a pending plastic write (pend), then
-// pend = 0. Bit 2 of status: the exponential series did not settle.
+// pend = 0. Sets *failed where the exponential series did not settle.
 __global__ void k_materialize_fp(int E, const double* __restrict__ Apend, int* __restrict__ pend,
-                                 const double* __restrict__ Fp_old, double* __restrict__ Fp, int* status) {
+                                 const double* __restrict__ Fp_old, double* __restrict__ Fp, int* failed) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < E; s += gridDim.x * blockDim.x) {
     if (!pend[s]) continue;
     const double a00 = Apend[0 * E + s], a11 = Apend[1 * E + s], a22 = Apend[2 * E + s];
     const double a01 = Apend[3 * E + s], a12 = Apend[4 * E + s], a02 = Apend[5 * E + s];
     const double Am[3][3] = {{a00, a01, a02}, {a01, a11, a12}, {a02, a12, a22}};
     double Ex[3][3];
-    if (!exp_traceless_sym(Am, Ex)) atomicOr(status, 2);
+    if (!exp_traceless_sym(Am, Ex)) *failed = 1;
     double Fo[3][3];
     for (int q = 0; q < 9; ++q) Fo[q / 3][q % 3] = Fp_old[q * E + s];
     for (int i = 0; i < 3; ++i)
@@ -1325,7 +1352,7 @@ struct RowSum {
 // the elements' diagonal records. ADJ stores the transpose (dR/du^T): block
 // (n, m) goes to block (m, n). The remaining blocks sum the nodal vectors, as
 // k_gather_nodes does (four threads per node, element order): R from the
-// records, and dM/du from dbuf if there is one.
+// records, and dM/du from dbuf, or zero without one.
 // The sums need no FP64 instruction but one conversion per matrix entry. At
 // 384,000 elements 231 us (3.9 TB/s; latency and the integer pipes, 47% busy)
 // against 268 us for the FP64 gathers, which the shorter element phase and the
@@ -1341,12 +1368,16 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
                                                      double* __restrict__ R, const double* __restrict__ dbuf,
                                                      double* __restrict__ dMdu) {
   if ((int)blockIdx.x >= row_blocks) {
-    const long long vectors = dbuf ? 2 : 1;
+    const long long vectors = 2;  // R, then dM/du
     for (long long t = (blockIdx.x - row_blocks) * (long long)blockDim.x + threadIdx.x; t < vectors * 4ll * N;
          t += (long long)(gridDim.x - row_blocks) * blockDim.x) {
       const bool second = t >= 4ll * N;
       const long long i = second ? t - 4ll * N : t;
       const int n = (int)(i >> 2), q = (int)(i & 3);
+      if (second && !dbuf) {  // no QoI: dM/du is cleared
+        dMdu[i] = 0.0;
+        continue;
+      }
       const double* src = second ? dbuf : reinterpret_cast<const double*>(rec);
       const int stride = second ? 16 : kRecord;
       double acc = 0.0;
@@ -1518,17 +1549,10 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
   }
 }
 
-double device_sum(const double* x, int n, DevBuf<double>& red, cudaStream_t st) {
+int reduction_blocks(Mechanics& m, int n) {
   const int nb = std::min(grid_for(n, 256), 1024);
-  if (red.n < 2 * (size_t)nb + 2) red.alloc(2 * nb + 2);
-  k_sum_partial<<<nb, 256, 0, st>>>(x, n, red.ptr);
-  GOAL_CHECK_LAUNCH();
-  k_sum_final<<<1, 1024, 0, st>>>(red.ptr, nb, red.ptr + 2 * nb);
-  GOAL_CHECK_LAUNCH();
-  double out = 0.0;
-  GOAL_CUDA(cudaMemcpyAsync(&out, red.ptr + 2 * nb, sizeof(double), cudaMemcpyDeviceToHost, st));
-  GOAL_CUDA(cudaStreamSynchronize(st));
-  return out;
+  if (m.red.n < 2 * (size_t)nb + 2) m.red.alloc(2 * nb + 2);
+  return nb;
 }
 
 }  // namespace
@@ -1568,8 +1592,9 @@ void Mechanics::init() {
   GOAL_CHECK_LAUNCH();
   refresh_cpinv();
   qoi_elem.alloc(E);
-  status.alloc(1);
-  status.zero(disc->stream);
+  ticket.alloc(1);
+  ticket.zero(disc->stream);
+  results.alloc();
 }
 
 void Mechanics::refresh_cpinv() {
@@ -1580,14 +1605,12 @@ void Mechanics::refresh_cpinv() {
 
 void Mechanics::materialize_fp() {
   const int E = disc->num_elems;
-  GOAL_CUDA(cudaMemsetAsync(status.ptr, 0, sizeof(int), disc->stream));
+  results.v->series = 0;
   k_materialize_fp<<<grid_for(E, 256), 256, 0, disc->stream>>>(E, st.Apend.ptr, st.pend.ptr, st.Fp_old.ptr, st.Fp.ptr,
-                                                               status.ptr);
+                                                               &results.v->series);
   GOAL_CHECK_LAUNCH();
-  int h = 0;
-  GOAL_CUDA(cudaMemcpyAsync(&h, status.ptr, sizeof(int), cudaMemcpyDeviceToHost, disc->stream));
   GOAL_CUDA(cudaStreamSynchronize(disc->stream));
-  GOAL_REQUIRE(h == 0, GOAL_ERR_RETURN_MAP, "J2: the exponential of the plastic increment did not converge");
+  GOAL_REQUIRE(!results.v->series, GOAL_ERR_RETURN_MAP, "J2: the exponential of the plastic increment did not converge");
 }
 
 void Mechanics::update_states() {
@@ -1610,18 +1633,15 @@ void SolInfo::init(Disc* d) {
 
 void ks_prepass(Mechanics& m, double rho, double& max_vm, double& scale, cudaStream_t st) {
   const int E = m.disc->num_elems;
-  const int nb = std::min(grid_for(E, 256), 1024);
-  if (m.red.n < 2 * (size_t)nb + 2) m.red.alloc(2 * nb + 2);
-  k_vm_max_partial<<<nb, 256, 0, st>>>(m.st.sigma.ptr, E, m.red.ptr);
+  const int nb = reduction_blocks(m, E);
+  double* mx = m.red.ptr + 2 * nb;
+  k_vm_max<<<nb, 256, 0, st>>>(m.st.sigma.ptr, E, m.red.ptr, m.ticket.ptr, mx, &m.results.v->max_vm);
   GOAL_CHECK_LAUNCH();
-  k_max_final<<<1, 1024, 0, st>>>(m.red.ptr, nb, m.red.ptr + 2 * nb);
+  k_ks_sum<<<nb, 256, 0, st>>>(m.st.sigma.ptr, m.disc->vol.ptr, E, rho, mx, m.red.ptr, m.ticket.ptr, &m.results.v->sum);
   GOAL_CHECK_LAUNCH();
-  k_ks_terms<<<grid_for(E, 256), 256, 0, st>>>(m.st.sigma.ptr, m.disc->vol.ptr, E, rho, m.red.ptr + 2 * nb,
-                                               m.qoi_elem.ptr);
-  GOAL_CHECK_LAUNCH();
-  GOAL_CUDA(cudaMemcpyAsync(&max_vm, m.red.ptr + 2 * nb, sizeof(double), cudaMemcpyDeviceToHost, st));
   GOAL_CUDA(cudaStreamSynchronize(st));
-  scale = device_sum(m.qoi_elem.ptr, E, m.red, st);
+  max_vm = m.results.v->max_vm;
+  scale = m.results.v->sum;
 }
 
 namespace {
@@ -1689,7 +1709,7 @@ double assemble(Mechanics& m, SolInfo* s, const Chain& c, const ErrorWeights* w,
   a.eqps = m.st.eqps.ptr;
   a.Apend = m.st.Apend.ptr;
   a.pend = m.st.pend.ptr;
-  a.status = m.status.ptr;
+  a.failed = &m.results.v->return_map;
   a.stab = m.stabilization ? 1 : 0;
   a.save = c.save_states;
   a.fp_reset = m.fp_reset ? 1 : 0;
@@ -1716,11 +1736,7 @@ double assemble(Mechanics& m, SolInfo* s, const Chain& c, const ErrorWeights* w,
   }
   a.ks_max = ks_max;
   a.ks_scale = ks_scale;
-  GOAL_CUDA(cudaMemsetAsync(m.status.ptr, 0, sizeof(int), st));
-  if (c.overwrite && c.jacobian && c.qoi == QOI_NONE && s) {  // zero_all also clears dMdu
-    // dMdu is not written by a chain without QoI: SolInfo::zero_all semantics
-    GOAL_CUDA(cudaMemsetAsync(s->dMdu.ptr, 0, sizeof(double) * s->dMdu.n, st));
-  }
+  m.results.v->return_map = 0;
   const bool buf = !c.colored && (c.mode != MODE_NONE || c.jacobian);
   const bool scatter = c.mode != MODE_NONE;
   const int E = d.num_elems;
@@ -1744,6 +1760,10 @@ double assemble(Mechanics& m, SolInfo* s, const Chain& c, const ErrorWeights* w,
       a.dbuf = m.dbuf.ptr;
     }
   }
+  if (c.overwrite && c.jacobian && c.qoi == QOI_NONE && s && !fix) {
+    // dMdu is not written by a chain without QoI: SolInfo::zero_all semantics (the fixed-point gather clears it)
+    GOAL_CUDA(cudaMemsetAsync(s->dMdu.ptr, 0, sizeof(double) * s->dMdu.n, st));
+  }
   const bool timed = g_phase.on;
   if (timed) GOAL_CUDA(cudaEventRecord(g_phase.ev[0], st));
   for (int e0 = 0; e0 < E; e0 += chunk) {
@@ -1758,7 +1778,7 @@ double assemble(Mechanics& m, SolInfo* s, const Chain& c, const ErrorWeights* w,
     if (fix) {
       const int rows = grid_for(d.num_nodes, 4, kSMs * 64);
       const bool dm = c.qoi != QOI_NONE;
-      const int nodes = grid_for((dm ? 8ll : 4ll) * d.num_nodes, 128, kSMs * 32);
+      const int nodes = grid_for(8ll * d.num_nodes, 128, kSMs * 32);
       auto gather = c.mode == MODE_ADJOINT ? k_gather_rows<true> : k_gather_rows<false>;
       gather<<<rows + nodes, 128, 0, st>>>(d.num_nodes, rows, d.brow_ptr.ptr, d.diag.ptr, d.btr.ptr, d.bptr.ptr,
                                            d.blist.ptr, d.nptr.ptr, d.nlist.ptr,
@@ -1805,15 +1825,15 @@ double assemble(Mechanics& m, SolInfo* s, const Chain& c, const ErrorWeights* w,
     }
   }
   if (timed) GOAL_CUDA(cudaEventRecord(g_phase.ev[2], st));
-  int hstat = 0;
-  GOAL_CUDA(cudaMemcpyAsync(&hstat, m.status.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
-  double q = 0.0;
-  if (c.qoi != QOI_NONE) {
-    q = device_sum(m.qoi_elem.ptr, d.num_elems, m.red, st);
-    if (c.qoi == QOI_KS_VM) q = ks_max + (1.0 / c.rho) * std::log(ks_scale);
-  } else {
-    GOAL_CUDA(cudaStreamSynchronize(st));
+  if (c.qoi == QOI_AVG_DISP) {
+    const int nb = reduction_blocks(m, E);
+    k_sum<<<nb, 256, 0, st>>>(m.qoi_elem.ptr, E, m.red.ptr, m.ticket.ptr, &m.results.v->sum);
+    GOAL_CHECK_LAUNCH();
   }
+  GOAL_CUDA(cudaStreamSynchronize(st));
+  double q = 0.0;
+  if (c.qoi == QOI_AVG_DISP) q = m.results.v->sum;
+  else if (c.qoi == QOI_KS_VM) q = ks_max + (1.0 / c.rho) * std::log(ks_scale);
   if (timed) {
     float e = 0.0f, g = 0.0f;
     GOAL_CUDA(cudaEventElapsedTime(&e, g_phase.ev[0], g_phase.ev[1]));
@@ -1822,7 +1842,7 @@ double assemble(Mechanics& m, SolInfo* s, const Chain& c, const ErrorWeights* w,
     g_phase.gather_ms += g;
     g_phase.count += 1;
   }
-  GOAL_REQUIRE(hstat == 0, GOAL_ERR_RETURN_MAP, "J2: return mapping failed");
+  GOAL_REQUIRE(!m.results.v->return_map, GOAL_ERR_RETURN_MAP, "J2: return mapping failed");
   return q;
 }
 

@@ -30,6 +30,27 @@ struct StatesDev {
   DevBuf<int> pend;
 };
 
+// Results that kernels write straight to host memory: the stream's
+// synchronization brings them, without a copy that has to be waited for too.
+struct HostResults {
+  struct Values {
+    int return_map;  // J2: the return map failed
+    int series;      // J2: the exponential of a plastic increment did not settle
+    double max_vm, sum;
+  };
+  Values* v = nullptr;
+  HostResults() = default;
+  HostResults(const HostResults&) = delete;
+  HostResults& operator=(const HostResults&) = delete;
+  ~HostResults() {
+    if (v) cudaFreeHost(v);
+  }
+  void alloc() {
+    if (!v) GOAL_CUDA(cudaHostAlloc(&v, sizeof(Values), cudaHostAllocMapped | cudaHostAllocPortable));
+    *v = Values{};
+  }
+};
+
 struct Mechanics {
   Disc* disc = nullptr;
   int model = MODEL_NEOHOOKEAN;
@@ -45,10 +66,11 @@ struct Mechanics {
   DevBuf<double> U;         // 4N nodal solution: u_x u_y u_z p per node (the DOF layout)
   StatesDev st;
   DevBuf<double> qoi_elem;  // E   per-element QoI values (colour order)
-  DevBuf<double> ebuf;      // two-phase assembly: per-element R and blocks (fixed-point records of 240 words, or 272 doubles)
+  DevBuf<double> ebuf;      // two-phase assembly: per-element R and blocks (records of 240 words, or 272 doubles)
   DevBuf<double> dbuf;      // two-phase assembly: per-element dM/du (16 doubles)
   DevBuf<double> red;       // reduction scratch
-  DevBuf<int> status;       // 1: return-map failures, non-finite etc.
+  DevBuf<unsigned> ticket;  // blocks that have finished a reduction (zero between reductions)
+  HostResults results;      // what the host reads after it has waited for the stream
   void init();
   void update_states();     // States::update (src/goal_states.cpp:130-141)
   void refresh_cpinv();
