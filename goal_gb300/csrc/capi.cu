@@ -230,8 +230,9 @@ int goal_disc_create(int num_nodes, int num_elems, const double* coords, const i
   GOAL_API_BEGIN
   GOAL_ARG(out && coords && tets && num_nodes > 0 && num_elems > 0, "goal_disc_create: bad arguments");
   GOAL_ARG(num_elem_sets >= 1, "goal_disc_create: need at least one element set");
-  for (long long i = 0; i < 4ll * num_elems; ++i)
-    GOAL_ARG(tets[i] >= 0 && tets[i] < num_nodes, "goal_disc_create: tet node out of range");
+  bool outside = false;
+  for (long long i = 0; i < 4ll * num_elems; ++i) outside |= (unsigned)tets[i] >= (unsigned)num_nodes;
+  GOAL_ARG(!outside, "goal_disc_create: tet node out of range");
   auto h = std::make_unique<goal_disc_s>();
   h->d = std::make_unique<Disc>();
   Disc& d = *h->d;

@@ -7,6 +7,7 @@
 #include <chrono>
 #include <cmath>
 
+#include "grid_barrier.cuh"
 #include "krylov.cuh"
 
 #include <cuda_fp16.h>

@@ -20,7 +20,6 @@
 
 constexpr int kCoopThreads = 512;            // worker threads of a CTA
 constexpr int kCoopWarps = kCoopThreads / 32;
-constexpr int kSpinLimit = 1 << 22;          // polls of a grid barrier (more than a second)
 
 template <typename T, typename TA, typename TV>
 struct CoopArgs {
@@ -58,11 +57,9 @@ __device__ __forceinline__ void givens_sync(int id) {
 }
 constexpr int kBarColumn = 2, kBarRotated = 3;  // a column is ready for the Givens warp; it has been rotated
 
-// The grid barrier: a counter of arrivals in global memory, waited for by one
-// thread of each CTA with a limit. 2,300 clocks among 152 CTAs; flags that
-// each CTA raises and all poll took 5,500 and more, and one cluster of 16 CTAs
-// that meet at an mbarrier gained nothing (its release waits for the same
-// stores).
+// The grid barrier (grid_barrier.cuh). Flags that each CTA raises and all poll
+// took 5,500 clocks and more against 2,300, and one cluster of 16 CTAs that
+// meet at an mbarrier gained nothing (its release waits for the same stores).
 struct CoopSync {
   unsigned* count;  // arrivals since the kernel began (cleared by the last CTA to leave)
   unsigned target;
@@ -71,15 +68,7 @@ struct CoopSync {
 
 // Warp 0 of every CTA, after a block barrier.
 __device__ __forceinline__ void coop_meet(CoopSync& s) {
-  if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(s.count) : "memory");
-    unsigned v;
-    int spins = 0;
-    do {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(s.count) : "memory");
-    } while (v < s.target && ++spins < kSpinLimit);
-    *s.ok = v >= s.target ? 1 : 0;
-  }
+  if (threadIdx.x == 0) *s.ok = grid_meet(s.count, s.target) ? 1 : 0;
   __syncwarp();
 }
 
