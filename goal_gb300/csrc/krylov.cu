@@ -1221,15 +1221,17 @@ template <typename T, typename TA, typename TV>
 void launch_coop(const CoopPlan& p, CoopArgs<T, TA, TV> a, int nnzb, cudaStream_t s) {
   const CoopDevice& d = coop_device();
   const size_t cap = 4 * (size_t)p.chunk, most = (size_t)d.smem;
+  auto pad = [](size_t bytes) { return (bytes + 31) / 32 * 32; };  // as the kernel lays them out
   // w, t, h, coefficients, scales, rotations, the reduction buffer, row pointers
-  const size_t fixed = 2 * sizeof(T) * cap + 12 * sizeof(T) * (size_t)(a.m + 2) + sizeof(T) * kCoopRed +
-                       sizeof(int) * (p.chunk + 1) + 640;
+  const size_t fixed = (a.Bc ? 2 : 1) * pad(sizeof(T) * cap) + 11 * pad(sizeof(T) * (a.m + 2)) +
+                       pad(sizeof(T) * kCoopRed) + pad(sizeof(int) * (p.chunk + 1));
   GOAL_REQUIRE(fixed <= most, GOAL_ERR_CAPACITY, "persistent cycle: rows per CTA exceed shared memory");
-  const size_t blocks = (a.Bc ? 2 : 1) * sizeof(T) * 4 * cap, basis = sizeof(TV) * (cap + 32) * (a.m + 1);
-  const size_t matrix = (size_t)(1.05 * p.chunk * nnzb / a.N) * (16 * sizeof(TA) + sizeof(int));
+  const size_t pitch = cap + (std::is_same<T, double>::value ? 1 : 32);
+  const size_t blocks = (a.Bc ? 2 : 1) * pad(sizeof(T) * 4 * cap), basis = pad(sizeof(TV) * pitch * (a.m + 1));
+  const size_t matrix = (size_t)(1.02 * p.chunk * nnzb / a.N) * (16 * sizeof(TA) + sizeof(int));  // rows differ
   // Shared memory for the basis and the matrix rows when both fit; what is
   // left out is read through L1, which is larger the less shared memory is asked for
-  size_t smem = fixed + blocks + 256;
+  size_t smem = fixed + blocks + 64;
   if (smem + basis + matrix <= most) smem = most;
   else if (smem + basis <= most / 2) smem += basis;
   a.chunk = p.chunk;
