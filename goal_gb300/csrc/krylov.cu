@@ -1200,18 +1200,21 @@ const CoopDevice& coop_device() {
 }
 
 // The persistent cycle wins while an Arnoldi step is bound by its launches and
-// its few blocks; past some 800 nodes to an SM the separate kernels, with more
-// threads in flight on the matrix and basis streams, are as fast. Whole solves
-// to 1e-12, ms, kernels -> persistent: FP64 343 nodes 26.5 -> 4.4, 9k 269 ->
-// 69, 24k 651 -> 261; binary16 inner 5k 28.0 -> 14.6, 36k 58 -> 36, 69k 88.5
-// -> 61.6, 118k 145 -> 126, 185k 230 -> 245 (learned 183 -> 247).
-// At least 8 nodes to a CTA: a warp of rows.
-constexpr int kCoopMinNodes = 8;
-constexpr int kCoopNodesPerSm = 800;
+// its few blocks; far enough up, the separate kernels with their more threads in
+// flight on the matrix and basis streams are faster, the earlier the more of a
+// step the products are. Whole solves to 1e-12, ms, kernels -> persistent:
+// binary16 inner 5k nodes 28.0 -> 11.3, 36k 58 -> 28, 59k 72.7 -> 44.4, 185k 230
+// -> 181, 275k 327 -> 303, 389k 520 -> 512, 531k 710 -> 781; with the second
+// sweep 149k 138 -> 109, 185k 182 -> 184, 227k 220 -> 234; binary32 133k 253 ->
+// 165, 227k 496 -> 329; FP64 inner 69k 318 -> 212, 133k 544 -> 469; FP64 343
+// 26.5 -> 3.9, 36k 1717 -> 828, 69k 5090 -> 3230 (not measured further up).
+constexpr int kCoopMinNodes = 8;  // of a CTA: a warp of rows
+constexpr int kCoopNodesPerSm = 2300, kCoopNodesPerSmSweep2 = 1150, kCoopNodesPerSmFp64 = 900;
 
-bool coop_plan(int N, CoopPlan& p) {
+bool coop_plan(int N, bool fp64, bool sweep2, CoopPlan& p) {
   const CoopDevice& d = coop_device();
-  if (N > kCoopNodesPerSm * d.sms) return false;
+  const int per_sm = fp64 ? kCoopNodesPerSmFp64 : sweep2 ? kCoopNodesPerSmSweep2 : kCoopNodesPerSm;
+  if (N > per_sm * d.sms) return false;
   p.chunk = std::max(kCoopMinNodes, (N + 8 * d.sms - 1) / (8 * d.sms) * 8);
   p.grid = (N + p.chunk - 1) / p.chunk;
   return true;
@@ -1304,7 +1307,7 @@ void issue_inner(const BsrView& A, long long n, int mi, bool sweep2, GState* st,
   const int nbx = vec_grid(n);
   cudaStream_t s = K.stream;
   CoopPlan plan;
-  if (coop_plan(N, plan)) {
+  if (coop_plan(N, std::is_same<T, double>::value, sweep2, plan)) {
     CoopArgs<T, TA, TV> a{};
     a.N = N;
     a.m = mi;
@@ -1445,7 +1448,7 @@ SolveStats fgmres(const BsrView& A, const double* vals, const double* b, double*
   const int batch = mixed ? 1 : 4;
 
   CoopPlan plan;
-  const bool coop = !mixed && coop_plan(N, plan);
+  const bool coop = !mixed && coop_plan(N, true, sweep2, plan);
   while (beta > tol_abs && out.iters < p.max_iters) {
     const int steps = std::min(m, p.max_iters - out.iters);
     int done_steps = 0;

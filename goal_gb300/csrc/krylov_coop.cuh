@@ -280,7 +280,7 @@ __device__ __forceinline__ double pow2_rsqrt(double x) {
 // lanes share a row group, each with every split-th column.
 template <typename T, typename TV>
 __device__ __forceinline__ T coop_update(T* w, const TV* V, long long vld, int rows, int ncols, const T* h,
-                                         int split) {
+                                         int split, bool staged) {
   constexpr int R = CoopRows<T>::R;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int per = 32 / split, gl = lane & (per - 1), s = lane / per;
@@ -292,13 +292,29 @@ __device__ __forceinline__ T coop_update(T* w, const TV* V, long long vld, int r
 #pragma unroll
     for (int e = 0; e < R; ++e) acc[e] = T(0);
     if (live) {
+      if (std::is_same<T, double>::value || staged) {
 #pragma unroll 4
-      for (int c = s; c < ncols; c += split) {
-        const T hc = h[c];
-        T v[R];
-        ld_rows<T, TV>(V + c * vld + g, v);
+        for (int c = s; c < ncols; c += split) {
+          const T hc = h[c];
+          T v[R];
+          ld_rows<T, TV>(V + c * vld + g, v);
 #pragma unroll
-        for (int e = 0; e < R; ++e) acc[e] = fma(hc, v[e], acc[e]);
+          for (int e = 0; e < R; ++e) acc[e] = fma(hc, v[e], acc[e]);
+        }
+      } else {  // from L2 or HBM: whole batches under way (64^3 mesh: 321 -> 301 ms a solve)
+        constexpr int B = 8;
+        for (int c0 = s; c0 < ncols; c0 += B * split) {
+          T v[B][R];
+#pragma unroll
+          for (int u = 0; u < B; ++u) ld_rows<T, TV>(V + min(c0 + u * split, ncols - 1) * vld + g, v[u]);
+#pragma unroll
+          for (int u = 0; u < B; ++u)
+            if (c0 + u * split < ncols) {
+              const T hc = h[c0 + u * split];
+#pragma unroll
+              for (int e = 0; e < R; ++e) acc[e] = fma(hc, v[u][e], acc[e]);
+            }
+        }
       }
     }
     for (int o = per; o < 32; o <<= 1)
@@ -687,7 +703,7 @@ __global__ void __launch_bounds__(kCoopThreads + 32, 1) k_gmres_coop(const CoopA
     if (!a.two_pass && cols > 0 && __ldcg(a.ctl)) break;
     coop_totals(a.part1, ldp, nc + 1, nc, scale, red, h1, coef);
     const T before = h1[nc];
-    T sq = coop_update<T, TV>(w, V, vld, rows, nc, coef, split);
+    T sq = coop_update<T, TV>(w, V, vld, rows, nc, coef, split, staged);
     const T* hs = h1;  // the projection that the norm estimate takes off
     bool second = false;
     if (a.two_pass) {
@@ -698,7 +714,7 @@ __global__ void __launch_bounds__(kCoopThreads + 32, 1) k_gmres_coop(const CoopA
       if (cols > 0 && __ldcg(a.ctl)) break;
       coop_totals(a.part2, ldp, nc + 1, nc, scale, red, h2, coef);
       second = h2[nc] < T(0.5) * before;
-      if (second) sq = coop_update<T, TV>(w, V, vld, rows, nc, coef, split);
+      if (second) sq = coop_update<T, TV>(w, V, vld, rows, nc, coef, split, staged);
       hs = h2;
     }
     if (tid < 32) {  // |w|^2 = |w before|^2 - |h|^2, enough for the storage scale
@@ -745,7 +761,7 @@ __global__ void __launch_bounds__(kCoopThreads + 32, 1) k_gmres_coop(const CoopA
   for (int c = tid; c < k; c += kCoopThreads) h1[c] = -scale[c] * __ldcg(a.y + c);
   for (int i = tid; i < rows; i += kCoopThreads) w[i] = T(0);
   coop_bar();
-  coop_update<T, TV>(w, V, vld, rows, k, h1, split);
+  coop_update<T, TV>(w, V, vld, rows, k, h1, split, staged);
   coop_bar();
   for (int i = tid; i < rows32; i += kCoopThreads) {
     const T u = block4(Dinv, i, i < rows ? w[i] : T(0));

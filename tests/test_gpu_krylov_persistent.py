@@ -67,3 +67,14 @@ def test_iteration_cap_and_zero_right_hand_side():
     assert st["iters"] == 17 and not st["converged"]
     x, st = api.solve(s, np.zeros_like(b), params=api.solve_params(tolerance=1e-10))
     assert st["converged"] and st["iters"] == 0 and not x.any()
+
+
+@pytest.mark.parametrize("precision,inner", [(api.MIXED, 60), (api.MIXED_F32, 23)])
+def test_basis_outside_shared_memory(precision, inner):
+    """Enough rows on a CTA that the basis and the matrix stay in device
+    memory, with column counts on both sides of a batch."""
+    d, m, s, A, b = _system(34, seed=3)
+    x, st = api.solve(s, b, params=api.solve_params(krylov_size=60, max_iters=20000, tolerance=1e-9,
+                                                    precision=precision, inner_iters=inner))
+    assert st["converged"]
+    assert np.linalg.norm(b - A @ x) <= 1.05e-9 * np.linalg.norm(b)
