@@ -140,8 +140,8 @@ struct Point {
 
 // Gather, kinematics, constitutive model with its state writes, and Mixed.
 template <int MODEL>
-__device__ __forceinline__ void eval_point(const ElemArgs& a, int s, const int (&v)[4], const double (&G)[4][3],
-                                           Point& p) {
+__device__ __forceinline__ void eval_point(const ElemArgs& a, bool save, int s, const int (&v)[4],
+                                           const double (&G)[4][3], Point& p) {
   const int E = a.d.num_elems;
   const double V = __ldg(a.d.vol + s);
   const int es = __ldg(a.d.elem_set + s);
@@ -263,7 +263,7 @@ __device__ __forceinline__ void eval_point(const ElemArgs& a, int s, const int (
       }
       gamma = 1.0 - 2.0 * mubar * Xr * rsmag;
       if (!(Xr >= 0.0) || !isfinite(Xr)) *a.failed = 1;
-      if (a.save) {
+      if (save) {
         a.eqps[s] = eq_old + sq23 * Xr;
         // Fp = exp(dgam N) Fp_old (stored only at plastic points): the
         // increment dgam N is stored here, Fp formed when it is read
@@ -276,7 +276,7 @@ __device__ __forceinline__ void eval_point(const ElemArgs& a, int s, const int (
         a.Apend[5 * E + s] = s02 * is;
         a.pend[s] = 1;
       }
-    } else if (a.save) {
+    } else if (save) {
       a.eqps[s] = eq_old;
       if (a.fp_reset) {
         a.pend[s] = 0;
@@ -299,7 +299,7 @@ __device__ __forceinline__ void eval_point(const ElemArgs& a, int s, const int (
     double dp = pval - pbar;
     sg[0][0] += dp; sg[1][1] += dp; sg[2][2] += dp;
   }
-  if (a.save) {
+  if (save) {
 #pragma unroll
     for (int q = 0; q < 9; ++q) a.sigma[q * E + s] = sg[q / 3][q % 3];
   }
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
 #pragma unroll
   for (int q = 0; q < 12; ++q) G[q / 3][q % 3] = __ldg(a.d.grads + q * E + s);
   Point pt;
-  eval_point<MODEL>(a, s, v, G, pt);
+  eval_point<MODEL>(a, a.save, s, v, G, pt);
   const double V = pt.V, inv_kappa = pt.inv_kappa, tau_coef = pt.tau_coef, pp_coef = pt.pp_coef;
   const double pval = pt.pval, J = pt.J, Jinv = pt.Jinv, alpha = pt.alpha, Ic3 = pt.Ic3;
   const double s00 = pt.s[0], s11 = pt.s[1], s22 = pt.s[2], s01 = pt.s[3], s12 = pt.s[4], s02 = pt.s[5];
@@ -662,25 +662,34 @@ __device__ __forceinline__ int off_index(int a, int b) { return 3 * a + b - (b >
 // with FP64 vectors m, q, n, X, Y, Z, now 432 (neo-Hookean 327). What bounds
 // it is latency at three warps per scheduler (registers and shared memory);
 // the FP64 pipe is 48% busy.
-constexpr int kFixThreads = 128;
+//
+// SPLIT threads in different warps share an element of a small mesh, where one
+// thread's chain of dependent instructions is all the time there is (36 us with
+// a warp alone on an SM): each forms the integration point, as the FP64 pipe
+// has room for that, its share of the four nodes and its share of the six block
+// pairs, to the same bits.
 constexpr int kFixC = 60, kFixW = 66, kFixSlots = 70;  // factors of h, q, X, Y, Z; c_ab; w_a
+constexpr int kFixNode = 70, kFixPart = 74, kFixSlotsSplit = 82;  // sizes of a node; F and the largest word of a part
+template <int ELEMS, int SPLIT>
+constexpr int kFixSmem = (SPLIT > 1 ? kFixSlotsSplit : kFixSlots) * ELEMS * (int)sizeof(long long);
 
-template <int MODEL>
-__global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
+template <int MODEL, int ELEMS, int SPLIT>
+__global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_fix(const ElemArgs a) {
   extern __shared__ long long fix_slots[];
-  const int s = a.begin + blockIdx.x * blockDim.x + threadIdx.x;
+  const int part = SPLIT > 1 ? threadIdx.x / ELEMS : 0;
+  const int s = a.begin + blockIdx.x * ELEMS + threadIdx.x % ELEMS;
   if (s >= a.end) return;
   const int E = a.d.num_elems;
-  long long* slot = fix_slots + threadIdx.x;
+  long long* slot = fix_slots + threadIdx.x % ELEMS;
   auto factor = [&](int i) {
-    const long long r = slot[i * kFixThreads];
+    const long long r = slot[i * ELEMS];
     Fx f;
     f.lo = (int)r;
     f.hi = (int)(r >> 32);
     return f;
   };
   auto put_factor = [&](int i, const Fx& f) {
-    slot[i * kFixThreads] = ((long long)f.hi << 32) | (unsigned)f.lo;
+    slot[i * ELEMS] = ((long long)f.hi << 32) | (unsigned)f.lo;
   };
   auto at = [](int v, int n, int k) { return 12 * v + 3 * n + k; };  // v: h q X Y Z
   double* rec_r = a.ebuf + (size_t)(s - a.ebase) * kRecord;
@@ -694,7 +703,7 @@ __global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
     double G[4][3];
 #pragma unroll
     for (int q = 0; q < 12; ++q) G[q / 3][q % 3] = __ldg(a.d.grads + q * E + s);
-    eval_point<MODEL>(a, s, v, G, pt);
+    eval_point<MODEL>(a, a.save && part == 0, s, v, G, pt);
   }
   const double V = pt.V, J = pt.J, Jinv = pt.Jinv, alpha = pt.alpha, Ic3 = pt.Ic3, gamma = pt.gamma;
   const double(&H)[3][3] = pt.H;
@@ -724,13 +733,13 @@ __global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
 #pragma unroll
     for (int i = 0; i < 3; ++i)
       ev += (((pt.un[0][i] * 0.25 + pt.un[1][i] * 0.25) + pt.un[2][i] * 0.25) + pt.un[3][i] * 0.25) * V;
-    a.qoi_elem[s] = ev * kThird;
+    if (part == 0) a.qoi_elem[s] = ev * kThird;
   } else if (a.qoi == QOI_KS_VM) {
     const double(&sg)[3][3] = pt.sg;
     double d1 = sg[0][0] - sg[1][1], d2 = sg[1][1] - sg[2][2], d3 = sg[2][2] - sg[0][0];
     double s7 = 0.5 * (d1 * d1 + d2 * d2 + d3 * d3 + 6.0 * (sg[0][1] * sg[0][1] + sg[1][2] * sg[1][2] + sg[2][0] * sg[2][0]));
     double ex = exp(a.rho * (sqrt(s7) - a.ks_max));
-    a.qoi_elem[s] = (1.0 / (a.rho * a.ks_scale)) * ex * V;
+    if (part == 0) a.qoi_elem[s] = (1.0 / (a.rho * a.ks_scale)) * ex * V;
     ks_w = (V / a.ks_scale) * ex;
   }
 
@@ -793,7 +802,7 @@ __global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
   unsigned long long bGs = 0;
   unsigned sh = 0, sq = 0, sx = 0, sy = 0;
 #pragma unroll 1
-  for (int n = 0; n < 4; ++n) {
+  for (int n = part; n < 4; n += SPLIT) {
     double G[3], hv[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) G[k] = __ldg(a.d.grads + (3 * n + k) * E + s);
@@ -834,8 +843,8 @@ __global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
       const long long qi = mi - fx_scale(c.value5(), bI - 1023);
       fq[i] = fx_split(qi);
       if (a.qoi == QOI_KS_VM) dM[i] = vq * fx_double(qi, xn) + vh * hv[i];
-      slot[at(0, n, i) * kFixThreads] = hi;
-      slot[at(1, n, i) * kFixThreads] = qi;
+      slot[at(0, n, i) * ELEMS] = hi;
+      slot[at(1, n, i) * ELEMS] = qi;
       mh |= fx_abs(hi);
       mq |= fx_abs(qi);
     }
@@ -863,9 +872,9 @@ __global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
       }
       Z.add(fzs, fh[k]);
       const long long x = X.value5(), y = Y.value5(), z = Z.value5();
-      slot[at(2, n, k) * kFixThreads] = x;
-      slot[at(3, n, k) * kFixThreads] = y;
-      slot[at(4, n, k) * kFixThreads] = z;
+      slot[at(2, n, k) * ELEMS] = x;
+      slot[at(3, n, k) * ELEMS] = y;
+      slot[at(4, n, k) * ELEMS] = z;
       mx |= fx_abs(x) | fx_abs(z);
       my |= fx_abs(y);
     }
@@ -873,6 +882,23 @@ __global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
     sq |= (unsigned)fx_bits(mq) << (8 * n);
     sx |= (unsigned)fx_bits(mx) << (8 * n);
     sy |= (unsigned)fx_bits(my) << (8 * n);
+    if (SPLIT > 1)
+      slot[(kFixNode + n) * ELEMS] = bG | (long long)fx_bits(mh) << 16 | (long long)fx_bits(mq) << 24 |
+                                     (long long)fx_bits(mx) << 32 | (long long)fx_bits(my) << 40;
+  }
+  if (SPLIT > 1) {
+    __syncthreads();
+    bGs = 0;
+    sh = sq = sx = sy = 0;
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const long long z = slot[(kFixNode + n) * ELEMS];
+      bGs |= (unsigned long long)(z & 0xffff) << (16 * n);
+      sh |= (unsigned)(z >> 16 & 255) << (8 * n);
+      sq |= (unsigned)(z >> 24 & 255) << (8 * n);
+      sx |= (unsigned)(z >> 32 & 255) << (8 * n);
+      sy |= (unsigned)(z >> 40 & 255) << (8 * n);
+    }
   }
 
   // The final scales. h_n: shifted to 62 bits, unit xl_n. X_n, Z_n: unit xl_n +
@@ -895,6 +921,10 @@ __global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
   // each would cost more)
 #pragma unroll 1
   for (int n = 0, p = 0; n < 3; ++n) {
+    if (SPLIT > 1 && n % SPLIT != part) {  // the pairs (n, b) are this node's
+      p += 3 - n;
+      continue;
+    }
     double G[3], CG[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) G[k] = __ldg(a.d.grads + (3 * n + k) * E + s);
@@ -913,7 +943,18 @@ __global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
       const double c = fma(CG[0], G[0], fma(CG[1], G[1], CG[2] * G[2]));
       all = max(all, fx_high(c));
       F = max(F, fx_exp(fx_high(c)) - 1146 - xl_of(n) - xl_of(b));
-      slot[(kFixC + p) * kFixThreads] = __double_as_longlong(c);
+      slot[(kFixC + p) * ELEMS] = __double_as_longlong(c);
+    }
+  }
+
+  if (SPLIT > 1) {
+    slot[(kFixPart + part) * ELEMS] = F;
+    slot[(kFixPart + 4 + part) * ELEMS] = all;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < SPLIT; ++k) {
+      F = max(F, (int)slot[(kFixPart + k) * ELEMS]);
+      all = max(all, (int)slot[(kFixPart + 4 + k) * ELEMS]);
     }
   }
 
@@ -935,18 +976,19 @@ __global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
   // h_n is in units 2^(exp_of(n) - 1082)
   auto exp_of = [&](int n) { return xl_of(n) + 1082; };
 #pragma unroll 1
-  for (int n = 0; n < 4; ++n) {
+  for (int n = part; n < 4; n += SPLIT) {
     const int dh = 62 - byte_of(sh, n), dx = dh + bX - 1023 - F, dy = dh + bY - 1023 - FY;
     long long w = 0;  // tau J V v . h_n
 #pragma unroll
     for (int q = 0; q < 15; ++q) {
       const int i = at(q / 3, n, q % 3);
-      const Fx f = fx_split(fx_scale(slot[i * kFixThreads], q < 3 ? dh : q < 6 ? dh + up : q >= 9 && q < 12 ? dy : dx));
+      const Fx f = fx_split(fx_scale(slot[i * ELEMS], q < 3 ? dh : q < 6 ? dh + up : q >= 9 && q < 12 ? dy : dx));
       put_factor(i, f);
       if (q < 3) w += fx_mul(ft[q], f);
     }
     put_factor(kFixW + n, fx_split(w));
   }
+  if (SPLIT > 1) __syncthreads();
 
   auto store_row = [&](long long* p, long long x0, long long x1, long long x2, long long x3) {
     st4(reinterpret_cast<double*>(p), __longlong_as_double(x0), __longlong_as_double(x1), __longlong_as_double(x2),
@@ -970,7 +1012,7 @@ __global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
     Fx hr[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) hr[k] = factor(at(0, r, k));
-    {  // column 3 of the diagonal block
+    if (SPLIT == 1 || r % SPLIT == part) {  // column 3 of the diagonal block
       const Fx e = fx_split(fx_mul(hr[0], hr[0]) + fx_mul(hr[1], hr[1]) + fx_mul(hr[2], hr[2]));
       int xpp;
       const long long pp = pp_block(e, er, er, xpp);
@@ -979,10 +1021,11 @@ __global__ void __launch_bounds__(kFixThreads, 3) k_elem_fix(const ElemArgs a) {
     }
 #pragma unroll 1
     for (int c = r + 1; c < 4; ++c, ++p) {
+      if (SPLIT > 1 && p % SPLIT != SPLIT - 1 - part) continue;
       const int ec = exp_of(c);
       const int x = er + ec + F - 2100;
       const long long cab =
-          fx_at(__longlong_as_double(slot[(kFixC + p) * kFixThreads]), x);
+          fx_at(__longlong_as_double(slot[(kFixC + p) * ELEMS]), x);
       Fx hc[3];
 #pragma unroll
       for (int k = 0; k < 3; ++k) hc[k] = factor(at(0, c, k));
@@ -1165,7 +1208,7 @@ __global__ void k_fill_identity(int E, double* Fp) {
 
 template <int MODEL, int MODE, bool JAC, bool ERR>
 void launch_colours(const Disc& d, ElemArgs args, cudaStream_t st, bool buffered) {
-  const int block = 128;
+  const int block = 64;  // 128 spreads less evenly: residual of 48k elements 44 us against 40, of 384k 256 both
   if (MODE == MODE_NONE || buffered) {
     // elements [args.begin, args.end) into the buffer (all of them, or a chunk)
     const int n = args.end - args.begin;
@@ -1184,6 +1227,14 @@ void launch_colours(const Disc& d, ElemArgs args, cudaStream_t st, bool buffered
   }
 }
 
+template <int MODEL, int ELEMS, int SPLIT>
+void launch_fix(const ElemArgs& args, int n, cudaStream_t st) {
+  constexpr int smem = kFixSmem<ELEMS, SPLIT>;
+  GOAL_CUDA(cudaFuncSetAttribute(k_elem_fix<MODEL, ELEMS, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  k_elem_fix<MODEL, ELEMS, SPLIT><<<(n + ELEMS - 1) / ELEMS, ELEMS * SPLIT, smem, st>>>(args);
+  GOAL_CHECK_LAUNCH();
+}
+
 template <int MODEL>
 void dispatch(const Disc& d, const Chain& c, const ElemArgs& args, cudaStream_t st, bool buf, bool fix) {
   if (c.error_chain) {
@@ -1192,10 +1243,17 @@ void dispatch(const Disc& d, const Chain& c, const ElemArgs& args, cudaStream_t 
     return;
   }
   if (fix) {
-    constexpr int smem = kFixSlots * kFixThreads * (int)sizeof(long long);
-    GOAL_CUDA(cudaFuncSetAttribute(k_elem_fix<MODEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    k_elem_fix<MODEL><<<(args.end - args.begin + kFixThreads - 1) / kFixThreads, kFixThreads, smem, st>>>(args);
-    GOAL_CHECK_LAUNCH();
+    // Four or two threads to an element while that is four warps to an SM (their
+    // FP64 work is repeated, so more would wait for its pipe: 10k elements with
+    // four 52 us, 16.5k with two 44); then blocks of 64 until there are two waves
+    // of 128, as they spread more evenly. J2, us, blocks of 128 -> now: 384 to
+    // 4.4k elements 40 -> 25, 6k 40 -> 29, 10k 40 -> 39.5, 25k 60 -> 51, 48k
+    // 82 -> 73; at 384k blocks of 64 take 435 against 432.
+    const int n = args.end - args.begin;
+    if (n <= 32 * kSMs) launch_fix<MODEL, 32, 4>(args, n, st);
+    else if (n <= 64 * kSMs) launch_fix<MODEL, 32, 2>(args, n, st);
+    else if (n <= 100000) launch_fix<MODEL, 64, 1>(args, n, st);
+    else launch_fix<MODEL, 128, 1>(args, n, st);
     return;
   }
   if (c.mode == MODE_NONE) {

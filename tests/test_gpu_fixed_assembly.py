@@ -96,3 +96,12 @@ def test_not_a_number_stays_where_it_was(mode):
     A, B = s.dRdu_csr(), z.dRdu_csr()
     assert np.isnan(B).any() and not np.isnan(B).all()
     assert np.array_equal(np.isnan(A), np.isnan(B)) and np.array_equal(np.isnan(s.R), np.isnan(z.R))
+
+
+@pytest.mark.parametrize("mode", [api.PRIMAL, api.ADJOINT])
+@pytest.mark.parametrize("n", [1, 2, 9, 10, 12, 26])
+def test_element_counts(n, mode):
+    """6 n^3 elements: four, two and one thread to an element, in blocks of 64
+    and of 128, the last block ragged."""
+    mesh = kuhn_cube(n, jitter=0.2, seed=n)
+    _close(*_both(mesh, api.J2, [J2], _state(mesh, 2e-3 / n, 8), mode))
