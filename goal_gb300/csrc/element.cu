@@ -131,7 +131,7 @@ __device__ bool exp_traceless_sym(const double A[3][3], double out[3][3]) {
 struct Point {
   double V, inv_kappa, tau_coef, pp_coef;
   double un[4][3], pval, gp[3];           // nodal displacements, pressure and its gradient
-  double J, Jinv, H[3][3], C[6], FC[3][3];
+  double J, Jinv, cof[3][3], H[3][3], C[6], FC[3][3];  // cof = J H, H = F^-T
   double alpha, Ic3, s[6];                // s: trial deviatoric Kirchhoff stress xx yy zz xy yz xz
   double gamma, smag, mubar, fyield, k0, cc, kh, rsmag, rcc;
   bool plastic;
@@ -146,7 +146,6 @@ __device__ __forceinline__ void eval_point(const ElemArgs& a, bool save, int s, 
   const double V = __ldg(a.d.vol + s);
   const int es = __ldg(a.d.elem_set + s);
   const double* mrow = a.mats + kMatStride * es;
-  const double kappa = __ldg(mrow + 0);
   const double mu = __ldg(mrow + 1);
   const double Kh = __ldg(mrow + 2);
   const double Yld = __ldg(mrow + 3);
@@ -244,23 +243,15 @@ __device__ __forceinline__ void eval_point(const ElemArgs& a, bool save, int s, 
       plastic = true;
       // reciprocals formed once (a division costs several FP64 instructions)
       rsmag = 1.0 / smag;
-      const double r2mu = 1.0 / (2.0 * mubar);
-      // first Newton iterate of src/goal_J2.cpp:101-121 (H = 0 in the first slope)
-      double X1 = fyield * r2mu;
-      double alpha1 = eq_old + sq23 * X1;
-      double R1 = smag - (2.0 * mubar * X1 + sq23 * (Yld + Kh * alpha1));
-      double r1 = fabs(R1);
-      // goal's tests |R| < 1e-11, |R|/Y < 1e-11, |R|/f < 1e-11 (Y, f > 0)
-      bool conv1 = (r1 < 1.0e-11) || (r1 < 1.0e-11 * Yld) || (r1 < 1.0e-11 * fyield);
-      kh = conv1 ? 0.0 : (2.0 / 3.0) * Kh;
-      cc = 2.0 * mubar + kh;
-      if (!conv1) {
-        rcc = 1.0 / cc;
-        Xr = fyield * rcc;
-      } else {
-        rcc = r2mu;  // cc = 2 mubar
-        Xr = X1;
-      }
+      // Newton iterates of src/goal_J2.cpp:101-121. The first has H = 0 in its
+      // slope, X1 = f / (2 mubar), and leaves the residual -2/3 K X1; goal stops
+      // there if |R| < 1e-11, |R|/Y < 1e-11 or |R|/f < 1e-11 (Y, f > 0).
+      const double m2 = 2.0 * mubar, K23 = (2.0 / 3.0) * Kh;
+      const bool conv1 = fabs(K23 * fyield) < 1.0e-11 * m2 * fmax(1.0, fmax(Yld, fyield));
+      kh = conv1 ? 0.0 : K23;
+      cc = m2 + kh;
+      rcc = 1.0 / cc;
+      Xr = fyield * rcc;
       gamma = 1.0 - 2.0 * mubar * Xr * rsmag;
       if (!(Xr >= 0.0) || !isfinite(Xr)) *a.failed = 1;
       if (save) {
@@ -287,18 +278,16 @@ __device__ __forceinline__ void eval_point(const ElemArgs& a, bool save, int s, 
   }
 
   // Cauchy stress of the model, then Mixed
-  const double pm = 0.5 * kappa * (J - Jinv);
+  // (the model's pressure 1/2 kappa (J - 1/J) is what Mixed takes out again,
+  // and with it what rounding left of the mean of s)
   const double gJ = gamma * Jinv;
   double sg[3][3];
-  sg[0][0] = s00 * gJ + pm; sg[1][1] = s11 * gJ + pm; sg[2][2] = s22 * gJ + pm;
+  sg[0][0] = s00 * gJ; sg[1][1] = s11 * gJ; sg[2][2] = s22 * gJ;
   sg[0][1] = sg[1][0] = s01 * gJ;
   sg[1][2] = sg[2][1] = s12 * gJ;
   sg[0][2] = sg[2][0] = s02 * gJ;
-  {
-    double pbar = ((sg[0][0] + sg[1][1]) + sg[2][2]) * kThird;
-    double dp = pval - pbar;
-    sg[0][0] += dp; sg[1][1] += dp; sg[2][2] += dp;
-  }
+  const double dp = fma(-kThird, (sg[0][0] + sg[1][1]) + sg[2][2], pval);
+  sg[0][0] += dp; sg[1][1] += dp; sg[2][2] += dp;
   if (save) {
 #pragma unroll
     for (int q = 0; q < 9; ++q) a.sigma[q * E + s] = sg[q / 3][q % 3];
@@ -314,7 +303,7 @@ __device__ __forceinline__ void eval_point(const ElemArgs& a, bool save, int s, 
   for (int i = 0; i < 3; ++i) {
     p.gp[i] = gp[i];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) { p.H[i][j] = H[i][j]; p.FC[i][j] = FC[i][j]; p.sg[i][j] = sg[i][j]; }
+    for (int j = 0; j < 3; ++j) { p.cof[i][j] = cof[i][j]; p.H[i][j] = H[i][j]; p.FC[i][j] = FC[i][j]; p.sg[i][j] = sg[i][j]; }
 #pragma unroll
     for (int q = 0; q < 4; ++q) p.un[q][i] = un[q][i];
   }
@@ -378,7 +367,43 @@ __global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
   // ---------------------------------------------------------------- residual
   if (MODE != MODE_NONE) {
     double Ru[4][3], Rp[4];
-    if (!ERR) {
+    if constexpr (!JAC && !ERR) {
+      // A residual alone, which the FP64 pipe bounds (all of its time): V J sigma
+      // F^-T = V sigma cof F, in the stabilization v . h_a with the cofactors on
+      // one side, and the last node from the others, as the gradients sum to
+      // zero: 102 FP64 instructions against 118 from h_a and J sigma, to the same
+      // error. (V gamma alpha (F C - Ic/3 F^-T) + p cof F would be 15 fewer, but
+      // the difference loses digits: error 1.3e-13 against 7e-14.) 384,000
+      // elements, J2, with the point's own 22 fewer: 257 us -> 234, neo-Hookean
+      // 194 -> 180.
+      const double rp0 = ((pval * inv_kappa) - dUdJ) * 0.25 * V;
+      double P[3][3], z[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          P[i][k] = (V * sg[i][0]) * pt.cof[0][k] + (V * sg[i][1]) * pt.cof[1][k] + (V * sg[i][2]) * pt.cof[2][k];
+      if (a.stab) {
+        const double f = tau * (V * Jinv);
+        double cg[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+          cg[i] = f * (pt.cof[i][0] * gp[0] + pt.cof[i][1] * gp[1] + pt.cof[i][2] * gp[2]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) z[k] = pt.cof[0][k] * cg[0] + pt.cof[1][k] * cg[1] + pt.cof[2][k] * cg[2];
+      }
+#pragma unroll
+      for (int n = 0; n < 3; ++n) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) Ru[n][i] = fma(P[i][0], G[n][0], fma(P[i][1], G[n][1], P[i][2] * G[n][2]));
+        Rp[n] = fma(z[0], G[n][0], fma(z[1], G[n][1], z[2] * G[n][2]));
+      }
+#pragma unroll
+      for (int i = 0; i < 3; ++i) Ru[3][i] = -((Ru[0][i] + Ru[1][i]) + Ru[2][i]);
+      Rp[3] = rp0 - ((Rp[0] + Rp[1]) + Rp[2]);
+#pragma unroll
+      for (int n = 0; n < 3; ++n) Rp[n] += rp0;
+    } else if constexpr (!ERR) {
       double TV[3][3];  // V J sigma
 #pragma unroll
       for (int q = 0; q < 9; ++q) TV[q / 3][q % 3] = V * T[q / 3][q % 3];
@@ -659,7 +684,7 @@ __device__ __forceinline__ int off_index(int a, int b) { return 3 * a + b - (b >
 // and the loops over nodes and pairs are not unrolled: unrolled, the kernel
 // was 12,800 instructions long and waited for instruction fetches 43% of the
 // time. J2 at 384,000 elements: 740 us in FP64 throughout, 1,208 unrolled, 498
-// with FP64 vectors m, q, n, X, Y, Z, now 432 (neo-Hookean 327). What bounds
+// with FP64 vectors m, q, n, X, Y, Z, now 422 (neo-Hookean 327). What bounds
 // it is latency at three warps per scheduler (registers and shared memory);
 // the FP64 pipe is 48% busy.
 //

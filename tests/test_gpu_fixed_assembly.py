@@ -105,3 +105,21 @@ def test_element_counts(n, mode):
     and of 128, the last block ragged."""
     mesh = kuhn_cube(n, jitter=0.2, seed=n)
     _close(*_both(mesh, api.J2, [J2], _state(mesh, 2e-3 / n, 8), mode))
+
+
+@pytest.mark.parametrize("model,K", [(api.NEOHOOKEAN, 1000.0), (api.J2, 1000.0), (api.J2, 0.0)])
+@pytest.mark.parametrize("n,scale", [(1, 1e-9), (5, 1e-3), (5, 0.02), (21, 1e-3)])
+def test_residual_alone(model, K, n, scale):
+    """The residual chain and the Jacobian chain form R from different products:
+    some hundred roundings of terms no larger than R's largest entries in a
+    state far from equilibrium, 1e-13 of them."""
+    mesh = kuhn_cube(n, jitter=0.2, seed=n)
+    d = api.Disc(mesh)
+    m = api.Mechanics(d, model, [[200e3, 0.3, K, 250.0, 1.0]])
+    m.set_solution(_state(mesh, scale / n, 9))
+    s, z = api.SolInfo(d), api.SolInfo(d)
+    api.assemble(m, s, api.PRIMAL, jacobian=True, save_states=False)
+    api.assemble(m, z, api.PRIMAL, jacobian=False, save_states=False)
+    A, B = s.R.reshape(-1, 4), z.R.reshape(-1, 4)
+    for c in (slice(0, 3), slice(3, 4)):
+        assert np.abs(A[:, c] - B[:, c]).max() <= 1e-13 * np.abs(A[:, c]).max()
