@@ -311,10 +311,39 @@ __device__ __forceinline__ void eval_point(const ElemArgs& a, bool save, int s, 
   for (int q = 0; q < 6; ++q) p.C[q] = C[q];
 }
 
+// The gather's launch overlaps the element phase: its blocks may be on the chip
+// by the time that phase ends, and wait there for its end and its stores. Chains
+// of 384 elements: Jacobian 42 us -> 39, residual 31 -> 28; J2 Jacobian of 384,000
+// 661 -> 658. A small element phase lets them come while it runs; waiting blocks
+// cost a chip full of element blocks more than they save (Jacobian of 48k 117 us
+// -> 126, of 384k 663 -> 753, residual of 48k 51 -> 60).
+__device__ __forceinline__ void gather_may_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+// The address that loads after the wait use, so that none can move ahead of it.
+template <typename T>
+__device__ __forceinline__ const T* wait_for_elements(const T* buffer) {
+  asm volatile("griddepcontrol.wait;" : "+l"(buffer)::"memory");
+  return buffer;
+}
+
+template <typename... P, typename... A>
+void launch_gather(void (*kernel)(P...), int grid, int block, cudaStream_t st, A... args) {
+  cudaLaunchAttribute overlap;
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = st;
+  cfg.attrs = &overlap;
+  cfg.numAttrs = 1;
+  GOAL_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 // BUF: element outputs go to the per-element buffer (phase 1 of the two-phase
 // assembly) instead of being accumulated in place by one colour at a time.
 template <int MODEL, int MODE, bool JAC, bool ERR, bool BUF>
 __global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
+  if (BUF && gridDim.x * blockDim.x <= 128 * kSMs) gather_may_start();
   const int s = a.begin + blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= a.end) return;
   const int E = a.d.num_elems;
@@ -701,6 +730,7 @@ constexpr int kFixSmem = (SPLIT > 1 ? kFixSlotsSplit : kFixSlots) * ELEMS * (int
 template <int MODEL, int ELEMS, int SPLIT>
 __global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_fix(const ElemArgs a) {
   extern __shared__ long long fix_slots[];
+  if (SPLIT > 1) gather_may_start();
   const int part = SPLIT > 1 ? threadIdx.x / ELEMS : 0;
   const int s = a.begin + blockIdx.x * ELEMS + threadIdx.x % ELEMS;
   if (s >= a.end) return;
@@ -1385,12 +1415,13 @@ __global__ void __launch_bounds__(256) k_gather_nodes(int N, const int* __restri
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < 4ll * N;
        t += (long long)gridDim.x * blockDim.x) {
     const int n = (int)(t >> 2), q = (int)(t & 3);
+    const int c0 = __ldg(nptr + n), c1 = __ldg(nptr + n + 1);
+    const double* buf = wait_for_elements(ebuf);
     double acc = accumulate ? out[t] : 0.0;
-    const int c1 = __ldg(nptr + n + 1);
-    for (int c = __ldg(nptr + n); c < c1; ++c) {
+    for (int c = c0; c < c1; ++c) {
       const int v = __ldg(nlist + c), e = v >> 2;
       if (e < lo || e >= hi) continue;
-      acc += __ldg(ebuf + (size_t)(e - lo) * estride + 4 * (v & 3) + q);
+      acc += __ldg(buf + (size_t)(e - lo) * estride + 4 * (v & 3) + q);
     }
     out[t] = acc;
   }
@@ -1457,16 +1488,16 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
       const bool second = t >= 4ll * N;
       const long long i = second ? t - 4ll * N : t;
       const int n = (int)(i >> 2), q = (int)(i & 3);
+      const int c0 = __ldg(nptr + n), c1 = __ldg(nptr + n + 1);
+      const double* src = wait_for_elements(second ? dbuf : reinterpret_cast<const double*>(rec));
       if (second && !dbuf) {  // no QoI: dM/du is cleared
         dMdu[i] = 0.0;
         continue;
       }
-      const double* src = second ? dbuf : reinterpret_cast<const double*>(rec);
       const int stride = second ? 16 : kRecord;
       double acc = 0.0;
-      const int c1 = __ldg(nptr + n + 1);
 #pragma unroll 4
-      for (int c = __ldg(nptr + n); c < c1; ++c) {
+      for (int c = c0; c < c1; ++c) {
         const int v = __ldg(nlist + c);
         acc += __ldg(src + (size_t)(v >> 2) * stride + 4 * (v & 3) + q);
       }
@@ -1485,6 +1516,8 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
     d[0] = odd ? t0 : a0; d[1] = odd ? a1 : t0; d[2] = odd ? t1 : a2; d[3] = odd ? a3 : t1;
   };
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  // no load below can be moved ahead of this: each is under the loop's condition
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   constexpr int kNone = -32768;  // exponent of no term: every shift takes it to zero
   __shared__ int lists[4][kRowTerms];
   int* mine = lists[threadIdx.x >> 5];
@@ -1863,19 +1896,16 @@ double assemble(Mechanics& m, SolInfo* s, const Chain& c, const ErrorWeights* w,
       const bool dm = c.qoi != QOI_NONE;
       const int nodes = grid_for(8ll * d.num_nodes, 128, kSMs * 32);
       auto gather = c.mode == MODE_ADJOINT ? k_gather_rows<true> : k_gather_rows<false>;
-      gather<<<rows + nodes, 128, 0, st>>>(d.num_nodes, rows, d.brow_ptr.ptr, d.diag.ptr, d.btr.ptr, d.bptr.ptr,
-                                           d.blist.ptr, d.nptr.ptr, d.nlist.ptr,
-                                           reinterpret_cast<const long long*>(m.ebuf.ptr), s->A.ptr, s->R.ptr,
-                                           dm ? m.dbuf.ptr : nullptr, s->dMdu.ptr);
-      GOAL_CHECK_LAUNCH();
+      launch_gather(gather, rows + nodes, 128, st, d.num_nodes, rows, d.brow_ptr.ptr, d.diag.ptr, d.btr.ptr, d.bptr.ptr,
+                    d.blist.ptr, d.nptr.ptr, d.nlist.ptr, reinterpret_cast<const long long*>(m.ebuf.ptr), s->A.ptr,
+                    s->R.ptr, dm ? m.dbuf.ptr : nullptr, s->dMdu.ptr);
       break;
     }
     const int acc = (c.overwrite && e0 == 0) ? 0 : 1;
     const bool chunked = chunk < E;
     if (scatter) {
-      k_gather_nodes<<<grid_for(4ll * d.num_nodes, 256), 256, 0, st>>>(d.num_nodes, d.nptr.ptr, d.nlist.ptr,
-                                                                          m.ebuf.ptr, a.estride, s->R.ptr, acc, e0, e1);
-      GOAL_CHECK_LAUNCH();
+      launch_gather(k_gather_nodes, grid_for(4ll * d.num_nodes, 256), 256, st, d.num_nodes, d.nptr.ptr, d.nlist.ptr,
+                    m.ebuf.ptr, a.estride, s->R.ptr, acc, e0, e1);
       if (c.jacobian) {
         const int noff = d.nnzb - d.num_nodes;
         const int* lists[2] = {d.offd.ptr, d.diag.ptr};
