@@ -337,6 +337,7 @@ void launch_gather(void (*kernel)(P...), int grid, int block, cudaStream_t st, A
   cfg.attrs = &overlap;
   cfg.numAttrs = 1;
   GOAL_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+  GOAL_CHECK_LAUNCH();
 }
 
 // BUF: element outputs go to the per-element buffer (phase 1 of the two-phase
@@ -715,7 +716,7 @@ __device__ __forceinline__ int off_index(int a, int b) { return 3 * a + b - (b >
 // time. J2 at 384,000 elements: 740 us in FP64 throughout, 1,208 unrolled, 498
 // with FP64 vectors m, q, n, X, Y, Z, now 422 (neo-Hookean 327). What bounds
 // it is latency at three warps per scheduler (registers and shared memory);
-// the FP64 pipe is 48% busy.
+// the FP64 pipe is 66% busy.
 //
 // SPLIT threads in different warps share an element of a small mesh, where one
 // thread's chain of dependent instructions is all the time there is (36 us with

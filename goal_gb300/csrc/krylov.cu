@@ -1194,7 +1194,7 @@ const CoopDevice& coop_device() {
     GOAL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     GOAL_REQUIRE(coop, GOAL_ERR_CUDA, "cooperative launches are not available");
     d.smem = optin - 512;  // the kernel's static shared memory stays below this
-    d.sms = std::min(sms, kCoopThreads);  // a thread polls one CTA's flag
+    d.sms = sms;
   }
   return d;
 }

@@ -15,8 +15,11 @@
 // Convergence is on the true (unpreconditioned) residual ||b - A x|| / ||b||,
 // which right preconditioning makes equal to the GMRES residual estimate.
 // Every iteration runs on the device (Arnoldi, classical Gram-Schmidt with a
-// conditional second pass, Givens rotations); the host reads one residual
-// estimate per outer iteration.
+// conditional second pass, Givens rotations). Systems within coop_plan's limits
+// run each inner cycle, or each cycle of a plain solve, as one cooperative
+// kernel (krylov_coop.cuh); larger ones and the outer iteration run a kernel per
+// step, gated on device state. The host reads the state once per outer iteration
+// (plain solves: once per cycle, or every few steps).
 #pragma once
 
 #include <cuda_fp16.h>

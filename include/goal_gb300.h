@@ -267,7 +267,8 @@ int goal_mechanics_device_solution(goal_mechanics m, double** U);
  * evaluates every element in one launch into a per-element buffer and then
  * sums each matrix block / nodal row over its incident elements in element
  * order; colored = 1 evaluates one colour (no two elements sharing a node) per
- * launch and accumulates in place, without the buffer (2176 bytes per element). */
+ * launch and accumulates in place, without the buffer (1920 bytes per element of
+ * an overwriting Jacobian chain, 2176 of an accumulating one). */
 typedef struct {
   int mode;
   int jacobian;
@@ -284,7 +285,7 @@ int goal_assemble(goal_mechanics m, goal_sol_info s, const goal_chain* chain, do
  * bytes; 16 more with a QoI). A mesh whose buffer would be larger is
  * assembled in chunks of elements, each evaluated into the buffer and then
  * added to the matrix and vectors; the sums and their order are those of one
- * pass, so the results are the same bits. 0 (default) = a quarter of the
+ * accumulating pass, so the results are the same bits as its. 0 (default) = a quarter of the
  * device's memory. Process-wide. */
 int goal_set_element_buffer_limit(long long bytes);
 /* No counterpart in the reference. Device time of goal_assemble's two phases,
