@@ -384,6 +384,54 @@ struct GivensShared {
   T beta;
 };
 
+// y = R^-1 g by one warp, column by column: entry r of g in lane r mod 32, D
+// columns of up to 32 Q rows in registers and D more on their way from L2. (One
+// column ahead, a step took L2's latency: 50k clocks for 60 columns, 5% of a
+// small cycle, while all CTAs wait for y.)
+template <typename T, int Q, int D>
+__device__ __forceinline__ void back_substitute(int k, const T* g, const T* dinv, const T* H, int ldh, T* y) {
+  const int lane = threadIdx.x & 31;
+  T gv[Q], dv[Q], c[D][Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int r = lane + 32 * q;
+    gv[q] = r < k ? g[r] : T(0);
+    dv[q] = r < k ? dinv[r] : T(0);
+  }
+  auto load = [&](T (&to)[D][Q], int top) {  // the entries above the diagonal of columns top, top - 1, ...
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        to[d][q] = lane + 32 * q < top - d ? H[(long long)ldh * (top - d) + lane + 32 * q] : T(0);
+  };
+  load(c, k - 1);
+  for (int top = k - 1; top >= 0; top -= D) {
+    T next[D][Q];
+    load(next, top - D);
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      const int i = top - d;
+      if (i < 0) break;
+      T gi = gv[0], di = dv[0];
+#pragma unroll
+      for (int q = 1; q < Q; ++q)
+        if (i >> 5 == q) {
+          gi = gv[q];
+          di = dv[q];
+        }
+      const T yi = __shfl_sync(0xffffffffu, gi * di, i & 31);
+      if (lane == (i & 31)) y[i] = yi;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) gv[q] -= c[d][q] * yi;
+    }
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+#pragma unroll
+      for (int q = 0; q < Q; ++q) c[d][q] = next[d][q];
+  }
+}
+
 template <typename T>
 __device__ void givens_warp(GivensShared<T>* gs, const T* col, T* rot, T* lows, T* cs, T* sn, T* g, T* dinv, T* H,
                             int ldh, T* y, double tol_abs, GState* st) {
@@ -438,30 +486,12 @@ __device__ void givens_warp(GivensShared<T>* gs, const T* col, T* rot, T* lows, 
     for (int i = lane; i <= j; i += 32) h[i] = rot[i];
     const bool done = gs->done != 0;
     if (done) {
-      // y = R^-1 g, column by column; the next column is loaded ahead
       const int k = j + 1;
-      T cur[kMaxM / 32], nxt[kMaxM / 32];
+      constexpr int D = std::is_same<T, double>::value ? 4 : 8;
       __syncwarp();
-#pragma unroll
-      for (int q = 0; q < kMaxM / 32; ++q) cur[q] = lane + 32 * q < k ? H[(long long)ldh * (k - 1) + lane + 32 * q] : T(0);
-      for (int i = k - 1; i >= 0; --i) {
-        if (i > 0) {
-#pragma unroll
-          for (int q = 0; q < kMaxM / 32; ++q)
-            nxt[q] = lane + 32 * q < i ? H[(long long)ldh * (i - 1) + lane + 32 * q] : T(0);
-        }
-        const T yi = g[i] * dinv[i];
-        __syncwarp();
-        if (lane == 0) y[i] = yi;
-#pragma unroll
-        for (int q = 0; q < kMaxM / 32; ++q) {
-          const int r = lane + 32 * q;
-          if (r < i) g[r] -= cur[q] * yi;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < kMaxM / 32; ++q) cur[q] = nxt[q];
-      }
+      if (k <= 64) back_substitute<T, 2, D>(k, g, dinv, H, ldh, y);
+      else if (k <= 128) back_substitute<T, 4, D / 2>(k, g, dinv, H, ldh, y);
+      else back_substitute<T, kMaxM / 32, D / 4>(k, g, dinv, H, ldh, y);
     }
     __syncwarp();
     givens_arrive(kBarRotated);
