@@ -14,6 +14,7 @@
 #include <chrono>
 
 #include "disc.cuh"
+#include "fixed.cuh"
 #include "grid_barrier.cuh"
 
 namespace goal {
@@ -244,7 +245,7 @@ __global__ void k_slots_and_min(int E, const int* tets, const int* brow_ptr, con
 __global__ void k_permute(int E, const int* perm, const int* tets, const int* elem_set, const int* color,
                           const int* blk_orig, const int* bmin, const int* nmin, const double* X,
                           int* tets_s, int* es_s, int* orig, int* pos, int* blk_s, unsigned* first,
-                          int* color_s, double* grads, double* vol, double* hh) {
+                          int* color_s, double* grads, double* vol, double* hh, int* flat) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < E; s += gridDim.x * blockDim.x) {
     int e = perm[s];
     orig[s] = e;
@@ -283,7 +284,13 @@ __global__ void k_permute(int E, const int* perm, const int* tets, const int* el
     Ji[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) / d;
     for (int a = 1; a < 4; ++a)
       for (int k = 0; k < 3; ++k) grads[(3 * a + k) * E + s] = Ji[a - 1][k];
-    for (int k = 0; k < 3; ++k) grads[k * E + s] = -(Ji[0][k] + Ji[1][k] + Ji[2][k]);
+    int axis[3];  // exponent of the largest gradient per axis
+    for (int k = 0; k < 3; ++k) {
+      const double g0 = -(Ji[0][k] + Ji[1][k] + Ji[2][k]);
+      grads[k * E + s] = g0;
+      axis[k] = max(max(fx_high(g0), fx_high(Ji[0][k])), max(fx_high(Ji[1][k]), fx_high(Ji[2][k]))) >> 20;
+    }
+    if (fx_spread(axis) > kFxSpread) atomicAdd(flat, 1);
     vol[s] = d / 6.0;
     const int ed[6][2] = {{0, 1}, {1, 2}, {0, 2}, {0, 3}, {1, 3}, {2, 3}};
     double hs = 0.0;
@@ -316,10 +323,12 @@ __global__ void k_contrib_keys(int E, const int* blk_s, const int* tets_s, int* 
   }
 }
 
-// color_ptr[c] = first position of a colour >= c in the sorted colours
+// color_ptr[c] = first position of a colour >= c in the sorted colours; behind
+// them a count that begins at zero
 __global__ void k_color_ptr(int E, const int* csorted, int* ptr) {
   const int c = threadIdx.x;
   if (c <= kMaxColors) ptr[c] = lower_bound_dev(csorted, E, c);
+  if (c == kMaxColors + 1) ptr[c] = 0;
 }
 
 // The build's temporary arrays, cut from one allocation (two dozen of their
@@ -471,11 +480,9 @@ void Disc::build() {
   int* perm = tmp.take(E);
   k_iota<<<grid_for(E, 256), 256, 0, s>>>(E, ids);
   sort_pairs(sc, ca, csorted, ids, perm, E, 8, s);
-  int* cptr = tmp.take(kMaxColors + 1);
+  int* cptr = tmp.take(kMaxColors + 2);
   k_color_ptr<<<1, 256, 0, s>>>(E, csorted, cptr);
   GOAL_CHECK_LAUNCH();
-  color_ptr.resize(kMaxColors + 1);
-  GOAL_CUDA(cudaMemcpyAsync(color_ptr.data(), cptr, sizeof(int) * (kMaxColors + 1), cudaMemcpyDeviceToHost, s));
 
   // block slots and first writers; the contribution lists' temporaries
   const int bbits = bits_for(nnzb);
@@ -505,9 +512,13 @@ void Disc::build() {
   h.alloc(E);
   k_permute<<<grid_for(E, 256), 256, 0, s>>>(E, perm, tets_o, es_o, ca, blk_orig, bmin, nmin, coords.ptr, tets.ptr, elem_set.ptr, elem_orig.ptr,
                                               elem_pos.ptr, blk.ptr, first.ptr, color.ptr, grads.ptr, vol.ptr,
-                                              h.ptr);
+                                              h.ptr, cptr + kMaxColors + 1);
   GOAL_CHECK_LAUNCH();
+  color_ptr.resize(kMaxColors + 2);
+  GOAL_CUDA(cudaMemcpyAsync(color_ptr.data(), cptr, sizeof(int) * (kMaxColors + 2), cudaMemcpyDeviceToHost, s));
+  GOAL_CUDA(cudaStreamSynchronize(s));
   phase(2);
+  flat_elems = color_ptr[kMaxColors + 1];
   // colours are numbered without gaps: the first one past the last colour starts at E
   num_colors = 0;
   while (num_colors < kMaxColors && color_ptr[num_colors] < E) ++num_colors;

@@ -73,6 +73,7 @@ struct Disc {
   // order, block slots, geometry), contribution lists, node and side sets
   double build_seconds[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   int color_rounds = 0;
+  int flat_elems = 0;  // elements that fixed point leaves to FP64 in any state (kFxSpread)
   cudaStream_t stream = nullptr;
 
   // host copies of the input (original element order)

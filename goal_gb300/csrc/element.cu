@@ -340,13 +340,22 @@ void launch_gather(void (*kernel)(P...), int grid, int block, cudaStream_t st, A
   GOAL_CHECK_LAUNCH();
 }
 
-// BUF: element outputs go to the per-element buffer (phase 1 of the two-phase
-// assembly) instead of being accumulated in place by one colour at a time.
-template <int MODEL, int MODE, bool JAC, bool ERR, bool BUF>
-__global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
-  if (BUF && gridDim.x * blockDim.x <= 128 * kSMs) gather_may_start();
-  const int s = a.begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= a.end) return;
+// Element record of the default Jacobian assembly, kRecord 8-byte words:
+//   [0, 16)    R (FP64)
+//   [16, 32)   per block (a, b) four 16-bit exponents: of K^uu, K^up, K^pu, K^pp
+//   [32, 48)   column 3 (K^up_a, K^pp_aa) of the diagonal blocks
+//   [48, 240)  the twelve off-diagonal blocks, row-major
+// with every block entry S 2^x in the fixed point of fixed.cuh, or in FP64 where
+// the exponent is kFxFloat.
+constexpr int kRecord = 240;
+constexpr int kRecExp = 16, kRecDiag = 32, kRecOff = 48;
+__device__ __forceinline__ int off_index(int a, int b) { return 3 * a + b - (b > a ? 1 : 0); }
+
+// One element in FP64. BUF: its outputs go to the per-element buffer (phase 1 of
+// the two-phase assembly) instead of being accumulated in place by one colour at
+// a time. REC: the buffer holds records (JAC && BUF).
+template <int MODEL, int MODE, bool JAC, bool ERR, bool BUF, bool REC>
+__device__ __forceinline__ void elem_fp64(const ElemArgs& a, bool save, int s) {
   const int E = a.d.num_elems;
 
   int v[4];
@@ -356,7 +365,7 @@ __global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
 #pragma unroll
   for (int q = 0; q < 12; ++q) G[q / 3][q % 3] = __ldg(a.d.grads + q * E + s);
   Point pt;
-  eval_point<MODEL>(a, a.save, s, v, G, pt);
+  eval_point<MODEL>(a, save, s, v, G, pt);
   const double V = pt.V, inv_kappa = pt.inv_kappa, tau_coef = pt.tau_coef, pp_coef = pt.pp_coef;
   const double pval = pt.pval, J = pt.J, Jinv = pt.Jinv, alpha = pt.alpha, Ic3 = pt.Ic3;
   const double s00 = pt.s[0], s11 = pt.s[1], s22 = pt.s[2], s01 = pt.s[3], s12 = pt.s[4], s02 = pt.s[5];
@@ -395,7 +404,7 @@ __global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
   for (int q = 0; q < 9; ++q) T[q / 3][q % 3] = J * sg[q / 3][q % 3];
 
   // ---------------------------------------------------------------- residual
-  if (MODE != MODE_NONE) {
+  if (MODE != MODE_NONE && !REC) {
     double Ru[4][3], Rp[4];
     if constexpr (!JAC && !ERR) {
       // A residual alone, which the FP64 pipe bounds (all of its time): V J sigma
@@ -633,7 +642,17 @@ __global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) K[3][k] = fma(pu1, hv[b][k], -fma(eab, tvv[k], twv[b] * hv[ai][k]));
     K[3][3] = fma(tJVs, eab, ppc);
-    if constexpr (BUF) {
+    if constexpr (REC) {
+      double* rec = a.ebuf + (size_t)(s - a.ebase) * kRecord;
+      if (ai == b) {
+        st4(rec + kRecDiag + 4 * ai, K[0][3], K[1][3], K[2][3], K[3][3]);
+      } else {
+        double* blk = rec + kRecOff + 16 * off_index(ai, b);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) st4(blk + 4 * r, K[r][0], K[r][1], K[r][2], K[r][3]);
+      }
+      reinterpret_cast<short4*>(rec + kRecExp)[4 * ai + b] = make_short4(kFxFloat, kFxFloat, kFxFloat, kFxFloat);
+    } else if constexpr (BUF) {
       double* eb = a.ebuf + (size_t)(s - a.ebase) * a.estride + 16 + 16 * (4 * ai + b);
 #pragma unroll
       for (int r = 0; r < 4; ++r) st4(eb + 4 * r, K[r][0], K[r][1], K[r][2], K[r][3]);
@@ -684,16 +703,20 @@ __global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
   }  // JAC
 }
 
+template <int MODEL, int MODE, bool JAC, bool ERR, bool BUF>
+__global__ void __launch_bounds__(128) k_elem(const ElemArgs a) {
+  if (BUF && gridDim.x * blockDim.x <= 128 * kSMs) gather_may_start();
+  const int s = a.begin + blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < a.end) elem_fp64<MODEL, MODE, JAC, ERR, BUF, false>(a, a.save, s);
+}
+
 // ------------------------------------------------------------------ fixed-point element phase
-// Element record of the default Jacobian assembly, kRecord 8-byte words:
-//   [0, 16)    R (FP64)
-//   [16, 32)   per block (a, b) four 16-bit exponents: of K^uu, K^up, K^pu, K^pp
-//   [32, 48)   column 3 (K^up_a, K^pp_aa) of the diagonal blocks
-//   [48, 240)  the twelve off-diagonal blocks, row-major
-// with every block entry S 2^x in the fixed point of fixed.cuh.
-constexpr int kRecord = 240;
-constexpr int kRecExp = 16, kRecDiag = 32, kRecOff = 48;
-__device__ __forceinline__ int off_index(int a, int b) { return 3 * a + b - (b > a ? 1 : 0); }
+// The record of an element that fixed point would hold to fewer digits than FP64
+// (see k_elem_fix). R, the QoI value and the states are written.
+template <int MODEL>
+__device__ __noinline__ void record_fp64(const ElemArgs& a, int s) {
+  elem_fp64<MODEL, MODE_PRIMAL, true, false, true, true>(a, false, s);
+}
 
 // Residual and tangent of one element per thread into its record, for both
 // Jacobian modes (the gather transposes).
@@ -710,6 +733,20 @@ __device__ __forceinline__ int off_index(int a, int b) { return 3 * a + b - (b >
 // linear in them), so k_gather_rows forms the diagonal blocks' u columns as
 // negated sums of the off-diagonal blocks.
 //
+// Every vector has its own exponent per node, so that its largest component
+// keeps 55 bits and more whatever the deformation: with one exponent for F C and
+// F^-T a block was off by 2e-12 of its largest entry at a dilation of 10 and by
+// all of it at 10,000 (now 2e-15 and 1e-14, as in FP64). What the exponents
+// cannot hold is left to FP64 (record_fp64): elements with an infinity or a NaN;
+// those whose F C G has fewer than kFixHeld bits, as |F C| |G| is far larger
+// (uniaxial stretches above 5); and those whose h differ by more than kFxSpread
+// exponents between the axes (flat elements, stretches above 30), as entries
+// that much smaller than the block's largest would lose digits of their own.
+// Against 113-bit arithmetic, over 60,000 random elements (sizes 1e-6 to 100,
+// strains 1e-9 to 1, dilations 0.1 to 1,000, stretches and flattenings to 100),
+// a block's largest error over its largest entry is at most 4 times FP64's, in
+// single blocks where those roundings happened to cancel, and the same over all.
+//
 // The factors wait in shared memory (a column of kFixSlots words per thread)
 // and the loops over nodes and pairs are not unrolled: unrolled, the kernel
 // was 12,800 instructions long and waited for instruction fetches 43% of the
@@ -723,13 +760,14 @@ __device__ __forceinline__ int off_index(int a, int b) { return 3 * a + b - (b >
 // a warp alone on an SM): each forms the integration point, as the FP64 pipe
 // has room for that, its share of the four nodes and its share of the six block
 // pairs, to the same bits.
-constexpr int kFixC = 60, kFixW = 66, kFixSlots = 70;  // factors of h, q, X, Y, Z; c_ab; w_a
-constexpr int kFixNode = 70, kFixPart = 74, kFixSlotsSplit = 82;  // sizes of a node; F and the largest word of a part
+constexpr int kFixC = 48, kFixW = 54, kFixNode = 58, kFixSlots = 62;  // factors of h, q, X, Y; c_ab; w_a; units of a node
+constexpr int kFixPart = 62, kFixSlotsSplit = 74;                     // scales and largest words of a part
+constexpr int kFixHeld = 55;
 template <int ELEMS, int SPLIT>
 constexpr int kFixSmem = (SPLIT > 1 ? kFixSlotsSplit : kFixSlots) * ELEMS * (int)sizeof(long long);
 
 template <int MODEL, int ELEMS, int SPLIT>
-__global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_fix(const ElemArgs a) {
+__global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_fix(const __grid_constant__ ElemArgs a) {
   extern __shared__ long long fix_slots[];
   if (SPLIT > 1) gather_may_start();
   const int part = SPLIT > 1 ? threadIdx.x / ELEMS : 0;
@@ -747,7 +785,7 @@ __global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_f
   auto put_factor = [&](int i, const Fx& f) {
     slot[i * ELEMS] = ((long long)f.hi << 32) | (unsigned)f.lo;
   };
-  auto at = [](int v, int n, int k) { return 12 * v + 3 * n + k; };  // v: h q X Y Z
+  auto at = [](int v, int n, int k) { return 12 * v + 3 * n + k; };  // v: h q X Y
   double* rec_r = a.ebuf + (size_t)(s - a.ebase) * kRecord;
   long long* rec = reinterpret_cast<long long*>(rec_r);
 
@@ -824,39 +862,38 @@ __global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_f
   const double zs = V * (ga * Ic3 - pJ), gaV = ga * V;
   const double upf = V * J * 0.25, ppc = V * pt.pp_coef, pu0 = V * ((J + Jinv) * 0.125);
 
-  // Fixed point from here on. Element scales: bL of F C and F^-T, bS of s, bX and
-  // bY of the coefficients of X, Z and of Y.
-  auto high3 = [](int l, const double(&x)[3][3]) {
+  // Fixed point from here on. Every factor has the exponent of its own kind: bF of
+  // F C, bS of s, bI of Ic/3, one for each coefficient, and per node bG and bh of
+  // the gradient and of h.
+  int lF = 0, lS = 0;
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
+  for (int i = 0; i < 3; ++i)
 #pragma unroll
-      for (int k = 0; k < 3; ++k) l = max(l, fx_high(x[i][k]));
-    return l;
-  };
-  int lS = 0;
+    for (int k = 0; k < 3; ++k) lF = max(lF, fx_high(FC[i][k]));
 #pragma unroll
   for (int q = 0; q < 6; ++q) lS = max(lS, fx_high(pt.s[q]));
-  const int lL = high3(high3(0, FC), H);
-  const int lX = max(max(fx_high(xm), fx_high(xh)), fx_high(zs)), lY = max(fx_high(yhc), fx_high(yqc));
-  int all = max(max(lL, max(lX, lY)), max(lS, max(fx_high(ync), fx_high(Ic3))));
-  const int bL = fx_exp(lL), bS = fx_exp(lS), bI = fx_exp(fx_high(Ic3));
-  const int bX = fx_exp(lX), bY = max(fx_exp(lY), need_n ? fx_exp(fx_high(ync)) + bS - 1020 : 0);
-  const int grow = max(bI - 1022, 0);
+  int all = max(max(lF, lS), max(max(fx_high(xm), fx_high(xh)), max(fx_high(zs), fx_high(Ic3))));
+  all = max(all, max(fx_high(yhc), max(fx_high(yqc), fx_high(ync))));
+  const int bF = fx_exp(lF), bS = fx_exp(lS), bI = fx_exp(fx_high(Ic3));
+  const int bm = fx_exp(fx_high(xm)), bp = fx_exp(fx_high(xh)), bz = fx_exp(fx_high(zs));
+  const int byh = fx_exp(fx_high(yhc)), byq = fx_exp(fx_high(yqc)), byn = fx_exp(fx_high(ync));
   Fx fFC[3][3], fS[6];
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int k = 0; k < 3; ++k) fFC[i][k] = fx_factor(FC[i][k], bL);
+    for (int k = 0; k < 3; ++k) fFC[i][k] = fx_factor(FC[i][k], bF);
 #pragma unroll
   for (int q = 0; q < 6; ++q) fS[q] = fx_factor(pt.s[q], bS);
-  const Fx fI = fx_factor(Ic3, bI), fxm = fx_factor(xm, bX), fxh = fx_factor(xh, bX), fzs = fx_factor(zs, bX);
-  const Fx fyh = fx_factor(yhc, bY), fyq = fx_factor(yqc, bY), fyn = fx_factor(ync, bY - bS + 1020);
+  const Fx fI = fx_factor62(Ic3, bI), fxm = fx_factor62(xm, bm), fxh = fx_factor62(xh, bp);
+  const Fx fyh = fx_factor62(yhc, byh), fyq = fx_factor62(yqc, byq), fyn = fx_factor62(ync, byn);
 
-  // Per node n, at the unit x_n = bL + bG_n + grow - 2101: h (from FP64, which R
-  // needs), m = F C G, q = m - Ic/3 h; X, Z at x_n + bX - 1023, Y at x_n + bY -
-  // 1023. Their largest sizes, packed 8 bits a node.
-  unsigned long long bGs = 0;
-  unsigned sh = 0, sq = 0, sx = 0, sy = 0;
+  // Per node n: h = F^-T G to 62 bits (from FP64, which R needs too), at the unit
+  // xh = bh - 1084; m = F C G at um; q = m - Ic/3 h, n = s m, X and Y each at the
+  // larger unit of its terms, so that none holds less of a term than FP64 would.
+  // The units less xh wait in 16 bits a node. F, FY, up: see below.
+  unsigned long long bhs = 0;
+  int axis[3] = {0, 0, 0};  // exponent of the largest h per axis
+  int F = bz - 1022, FY = -32768, up = 32767, held = 64;
 #pragma unroll 1
   for (int n = part; n < 4; n += SPLIT) {
     double G[3], hv[3];
@@ -874,34 +911,35 @@ __global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_f
       st4(a.dbuf + 16ll * (s - a.ebase) + 4 * n, d, d, d, 0.0);
     }
     const int lG = max(fx_high(G[0]), max(fx_high(G[1]), fx_high(G[2]))), bG = fx_exp(lG);
-    all = max(max(all, lG), max(fx_high(hv[0]), max(fx_high(hv[1]), fx_high(hv[2]))));
-    bGs |= (unsigned long long)bG << (16 * n);
-    const int xn = bL + bG + grow - 2101;
+    const int lh = max(fx_high(hv[0]), max(fx_high(hv[1]), fx_high(hv[2]))), bh = fx_exp(lh);
+    all = max(all, max(lG, lh));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) axis[k] = max(axis[k], fx_high(hv[k]) >> 20);
+    const int um = bF + bG - 2103, uP = bI + bh - 2104, uq = max(um, uP), un = um + bS - 1021;
+    const int uX = max(bm + um - 1021, bp + bh - 2105);
+    const int uY = max(byh + bh - 2105, need_n ? max(byq + uq - 1021, byn + un - 1021) : -32768);
     Fx fG[3], fm[3], fh[3], fq[3], fn[3];
     double dM[3];  // d (KS) / du = vq q + vh h + vn n
 #pragma unroll
     for (int k = 0; k < 3; ++k) fG[k] = fx_factor(G[k], bG);
-    unsigned long long mh = 0, mq = 0, mx = 0, my = 0;
+    unsigned long long mm = 0, mq = 0, mX = 0, mY = 0;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      FxSum m, c;
+      FxSum m;
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         m.add(fFC[i][k], fG[k]);
         m.add_low(fFC[i][k], fG[k]);
       }
-      const int down = min(4 + grow, 62);
-      const long long mi = (m.value5() + (1ll << (down - 1))) >> down, hi = fx_at(hv[i], xn);
+      const long long mi = (m.value<5>() + 2) >> 2;
       fm[i] = fx_split(mi);
-      fh[i] = fx_split(hi);
-      c.add(fI, fh[i]);
-      c.add_low(fI, fh[i]);
-      const long long qi = mi - fx_scale(c.value5(), bI - 1023);
+      fh[i] = fx_factor62(hv[i], bh);
+      const long long qi = (mi >> fx_shift(uq - um)) - (fx_mul(fI, fh[i]) >> fx_shift(uq - uP));
       fq[i] = fx_split(qi);
-      if (a.qoi == QOI_KS_VM) dM[i] = vq * fx_double(qi, xn) + vh * hv[i];
-      slot[at(0, n, i) * ELEMS] = hi;
+      if (a.qoi == QOI_KS_VM) dM[i] = vq * fx_double(qi, uq) + vh * hv[i];
+      put_factor(at(0, n, i), fh[i]);
       slot[at(1, n, i) * ELEMS] = qi;
-      mh |= fx_abs(hi);
+      mm |= fx_abs(mi);
       mq |= fx_abs(qi);
     }
     if (need_n) {
@@ -909,70 +947,48 @@ __global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_f
       n0.add(fS[0], fm[0]); n0.add(fS[3], fm[1]); n0.add(fS[5], fm[2]);
       n1.add(fS[3], fm[0]); n1.add(fS[1], fm[1]); n1.add(fS[4], fm[2]);
       n2.add(fS[5], fm[0]); n2.add(fS[4], fm[1]); n2.add(fS[2], fm[2]);
-      const long long nv[3] = {n0.value5() >> 3, n1.value5() >> 3, n2.value5() >> 3};
+      const long long nv[3] = {n0.value<4>() >> 1, n1.value<4>() >> 1, n2.value<4>() >> 1};
 #pragma unroll
       for (int k = 0; k < 3; ++k) fn[k] = fx_split(nv[k]);
       if (a.qoi == QOI_KS_VM)
-        st4(a.dbuf + 16ll * (s - a.ebase) + 4 * n, dM[0] + vn * fx_double(nv[0], xn + bS - 1020),
-            dM[1] + vn * fx_double(nv[1], xn + bS - 1020), dM[2] + vn * fx_double(nv[2], xn + bS - 1020), 0.0);
+        st4(a.dbuf + 16ll * (s - a.ebase) + 4 * n, dM[0] + vn * fx_double(nv[0], un),
+            dM[1] + vn * fx_double(nv[1], un), dM[2] + vn * fx_double(nv[2], un), 0.0);
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      FxSum X, Y, Z;
-      X.add(fxm, fm[k]);
-      X.add(fxh, fh[k]);
-      Y.add(fyh, fh[k]);
-      if (need_n) {
-        Y.add(fyq, fq[k]);
-        Y.add(fyn, fn[k]);
-      }
-      Z.add(fzs, fh[k]);
-      const long long x = X.value5(), y = Y.value5(), z = Z.value5();
+      const long long x = (fx_mul1(fxm, fm[k]) >> fx_shift(uX - (bm + um - 1021))) +
+                          (fx_mul1(fxh, fh[k]) >> fx_shift(uX - (bp + bh - 2105)));
+      long long y = fx_mul1(fyh, fh[k]) >> fx_shift(uY - (byh + bh - 2105));
+      if (need_n)
+        y += (fx_mul1(fyq, fq[k]) >> fx_shift(uY - (byq + uq - 1021))) +
+             (fx_mul1(fyn, fn[k]) >> fx_shift(uY - (byn + un - 1021)));
       slot[at(2, n, k) * ELEMS] = x;
       slot[at(3, n, k) * ELEMS] = y;
-      slot[at(4, n, k) * ELEMS] = z;
-      mx |= fx_abs(x) | fx_abs(z);
-      my |= fx_abs(y);
+      mX |= fx_abs(x);
+      mY |= fx_abs(y);
     }
-    sh |= (unsigned)fx_bits(mh) << (8 * n);
-    sq |= (unsigned)fx_bits(mq) << (8 * n);
-    sx |= (unsigned)fx_bits(mx) << (8 * n);
-    sy |= (unsigned)fx_bits(my) << (8 * n);
-    if (SPLIT > 1)
-      slot[(kFixNode + n) * ELEMS] = bG | (long long)fx_bits(mh) << 16 | (long long)fx_bits(mq) << 24 |
-                                     (long long)fx_bits(mx) << 32 | (long long)fx_bits(my) << 40;
+    const int unit = bh - 1084, rq = uq - unit, rX = uX - unit, rY = uY - unit;
+    held = min(held, fx_bits(mm));
+    up = min(up, 62 - rq - fx_bits(mq));
+    F = max(F, rX + fx_bits(mX) - 62);
+    FY = max(FY, rY + fx_bits(mY) - 62);
+    bhs |= (unsigned long long)bh << (16 * n);
+    slot[(kFixNode + n) * ELEMS] =
+        (long long)rY << 48 | (long long)(rX & 0xffff) << 32 | (long long)(rq & 0xffff) << 16 | bh;
   }
   if (SPLIT > 1) {
     __syncthreads();
-    bGs = 0;
-    sh = sq = sx = sy = 0;
+    bhs = 0;
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const long long z = slot[(kFixNode + n) * ELEMS];
-      bGs |= (unsigned long long)(z & 0xffff) << (16 * n);
-      sh |= (unsigned)(z >> 16 & 255) << (8 * n);
-      sq |= (unsigned)(z >> 24 & 255) << (8 * n);
-      sx |= (unsigned)(z >> 32 & 255) << (8 * n);
-      sy |= (unsigned)(z >> 40 & 255) << (8 * n);
-    }
+    for (int n = 0; n < 4; ++n) bhs |= (unsigned long long)(slot[(kFixNode + n) * ELEMS] & 0xffff) << (16 * n);
   }
 
-  // The final scales. h_n: shifted to 62 bits, unit xl_n. X_n, Z_n: unit xl_n +
-  // F. q_n is far smaller than h_n near the undeformed state and a plastic Y_n
-  // far larger than X_n, so they have their own: q_n unit xl_n - up, Y_n unit
-  // xl_n + FY; their products come `down` bits finer than the others.
-  auto byte_of = [](unsigned x, int n) { return (int)((x >> (8 * n)) & 255u); };
-  auto bG_of = [&](int n) { return (int)(bGs >> (16 * n)) & 0xffff; };
-  auto xl_of = [&](int n) { return bL + bG_of(n) + grow - 2163 + byte_of(sh, n); };
-  int F = -32768, FY = -32768, up = 32767;
-#pragma unroll 1
-  for (int n = 0; n < 4; ++n) {
-    const int h0 = 1022 + byte_of(sh, n);
-    F = max(F, bX - h0 - 1 + byte_of(sx, n));
-    FY = max(FY, bY - h0 - 1 + byte_of(sy, n));
-    up = min(up, byte_of(sh, n) - byte_of(sq, n));
-  }
-  F = max(F, FY - up);
+  // The final scales. X_n, Z_n: unit xh_n + F. q_n is far smaller than h_n near the
+  // undeformed state and a plastic Y_n far larger than X_n, so they have their own:
+  // q_n unit xh_n - up, Y_n unit xh_n + FY; their products come `down` bits finer
+  // than the others.
+  auto of16 = [](long long w, int n) { return (int)(short)(w >> (16 * n)); };
+  auto xh_of = [&](int n) { return of16(bhs, n) - 1084; };
   // c_ab = ga V G_a . C G_b of the pairs (in FP64: two numbers to quantize for
   // each would cost more)
 #pragma unroll 1
@@ -998,21 +1014,31 @@ __global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_f
       for (int k = 0; k < 3; ++k) G[k] = __ldg(a.d.grads + (3 * b + k) * E + s);
       const double c = fma(CG[0], G[0], fma(CG[1], G[1], CG[2] * G[2]));
       all = max(all, fx_high(c));
-      F = max(F, fx_exp(fx_high(c)) - 1146 - xl_of(n) - xl_of(b));
+      F = max(F, fx_exp(fx_high(c)) - 1146 - xh_of(n) - xh_of(b));
       slot[(kFixC + p) * ELEMS] = __double_as_longlong(c);
     }
   }
 
   if (SPLIT > 1) {
-    slot[(kFixPart + part) * ELEMS] = F;
-    slot[(kFixPart + 4 + part) * ELEMS] = all;
+    slot[(kFixPart + part) * ELEMS] = ((long long)held << 32) | (unsigned)all;
+    slot[(kFixPart + 4 + part) * ELEMS] = ((long long)F << 32) | ((long long)(FY & 0xffff) << 16) | (up & 0xffff);
+    slot[(kFixPart + 8 + part) * ELEMS] = ((long long)axis[0] << 32) | ((long long)axis[1] << 16) | axis[2];
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < SPLIT; ++k) {
-      F = max(F, (int)slot[(kFixPart + k) * ELEMS]);
-      all = max(all, (int)slot[(kFixPart + 4 + k) * ELEMS]);
+      const long long z = slot[(kFixPart + k) * ELEMS], f = slot[(kFixPart + 4 + k) * ELEMS];
+      held = min(held, (int)(z >> 32));
+      all = max(all, (int)z);
+      F = max(F, (int)(f >> 32));
+      FY = max(FY, (int)(short)(f >> 16));
+      up = min(up, (int)(short)f);
+      const long long x = slot[(kFixPart + 8 + k) * ELEMS];
+      axis[0] = max(axis[0], (int)(x >> 32));
+      axis[1] = max(axis[1], (int)(x >> 16 & 0xffff));
+      axis[2] = max(axis[2], (int)(x & 0xffff));
     }
   }
+  F = max(F, FY - up);
 
   // scales of the other entries, and the factors
   double tvv[3];
@@ -1022,37 +1048,41 @@ __global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_f
   const int bT = fx_exp(lt), bJ = fx_exp(fx_high(tJV)), bU = fx_exp(fx_high(upf));
   const int bP = fx_exp(fx_high(pu0)), xc = fx_exp(fx_high(ppc)) - 1082;
   all = max(max(all, lt), max(max(fx_high(tJV), fx_high(upf)), max(fx_high(pu0), fx_high(ppc))));
-  const bool bad = all >= 0x7ff00000;
-  const Fx fJ = fx_factor62(tJV, bJ), fU = fx_factor62(upf, bU), fP = fx_factor62(pu0, bP);
+  const bool wide = all >= 0x7ff00000 || held < kFixHeld || fx_spread(axis) > kFxSpread;
+  const Fx fz = fx_factor62(zs, bz), fJ = fx_factor62(tJV, bJ), fU = fx_factor62(upf, bU), fP = fx_factor62(pu0, bP);
   const long long mass = fx_at(ppc, xc);
   Fx ft[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) ft[k] = fx_factor62(tvv[k], bT);
   const int down = F + up - FY;
   // h_n is in units 2^(exp_of(n) - 1082)
-  auto exp_of = [&](int n) { return xl_of(n) + 1082; };
+  auto exp_of = [&](int n) { return of16(bhs, n) - 2; };
 #pragma unroll 1
   for (int n = part; n < 4; n += SPLIT) {
-    const int dh = 62 - byte_of(sh, n), dx = dh + bX - 1023 - F, dy = dh + bY - 1023 - FY;
+    const long long units = slot[(kFixNode + n) * ELEMS];
+    const int dq = of16(units, 1) + up, dX = of16(units, 2) - F, dY = of16(units, 3) - FY;
     long long w = 0;  // tau J V v . h_n
 #pragma unroll
-    for (int q = 0; q < 15; ++q) {
+    for (int q = 0; q < 3; ++q) w += fx_mul(ft[q], factor(at(0, n, q)));
+#pragma unroll
+    for (int q = 3; q < 12; ++q) {
       const int i = at(q / 3, n, q % 3);
-      const Fx f = fx_split(fx_scale(slot[i * ELEMS], q < 3 ? dh : q < 6 ? dh + up : q >= 9 && q < 12 ? dy : dx));
-      put_factor(i, f);
-      if (q < 3) w += fx_mul(ft[q], f);
+      put_factor(i, fx_split(fx_scale(slot[i * ELEMS], q < 6 ? dq : q < 9 ? dX : dY)));
     }
     put_factor(kFixW + n, fx_split(w));
   }
   if (SPLIT > 1) __syncthreads();
+  if (wide) {
+    if (part == 0) record_fp64<MODEL>(a, s);
+    return;
+  }
 
   auto store_row = [&](long long* p, long long x0, long long x1, long long x2, long long x3) {
     st4(reinterpret_cast<double*>(p), __longlong_as_double(x0), __longlong_as_double(x1), __longlong_as_double(x2),
         __longlong_as_double(x3));
   };
   auto store_exps = [&](int r, int c, int uu, int up, int pu, int pp) {
-    reinterpret_cast<short4*>(rec + kRecExp)[4 * r + c] =
-        bad ? make_short4(kFxBad, kFxBad, kFxBad, kFxBad) : make_short4((short)uu, (short)up, (short)pu, (short)pp);
+    reinterpret_cast<short4*>(rec + kRecExp)[4 * r + c] = make_short4((short)uu, (short)up, (short)pu, (short)pp);
   };
   // e_ab = h_a . h_b, and K^pp: the pressure mass term and tau J e_ab at a common scale
   auto pp_block = [&](const Fx& e, int er, int ec, int& x) {
@@ -1068,12 +1098,15 @@ __global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_f
     Fx hr[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) hr[k] = factor(at(0, r, k));
+    Fx Z[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) Z[k] = fx_split(fx_scale(fx_mul1(fz, hr[k]), bz - 1021 - F));
     if (SPLIT == 1 || r % SPLIT == part) {  // column 3 of the diagonal block
       const Fx e = fx_split(fx_mul(hr[0], hr[0]) + fx_mul(hr[1], hr[1]) + fx_mul(hr[2], hr[2]));
       int xpp;
       const long long pp = pp_block(e, er, er, xpp);
-      store_row(rec + kRecDiag + 4 * r, fx_mul(fU, hr[0]), fx_mul(fU, hr[1]), fx_mul(fU, hr[2]), pp);
-      store_exps(r, r, kFxBad, bU + er - 2102, kFxBad, xpp);
+      store_row(rec + kRecDiag + 4 * r, fx_mul1(fU, hr[0]), fx_mul1(fU, hr[1]), fx_mul1(fU, hr[2]), pp);
+      store_exps(r, r, 0, bU + er - 2103, 0, xpp);
     }
 #pragma unroll 1
     for (int c = r + 1; c < 4; ++c, ++p) {
@@ -1087,11 +1120,9 @@ __global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_f
       for (int k = 0; k < 3; ++k) hc[k] = factor(at(0, c, k));
       long long P[3][3];  // h_c Z_r + c_ab I: shared by the pair
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const Fx z = factor(at(4, r, k));
+      for (int k = 0; k < 3; ++k)
 #pragma unroll
-        for (int i = 0; i < 3; ++i) P[i][k] = fx_mul(hc[i], z) + (i == k ? cab : 0);
-      }
+        for (int i = 0; i < 3; ++i) P[i][k] = fx_mul(hc[i], Z[k]) + (i == k ? cab : 0);
       const Fx e = fx_split(fx_mul(hr[0], hc[0]) + fx_mul(hr[1], hc[1]) + fx_mul(hr[2], hc[2]));
       const Fx wr = factor(kFixW + r), wc = factor(kFixW + c);
       int xpp;
@@ -1120,7 +1151,7 @@ __global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_f
           for (int k = 0; k < 3; ++k) {
             K[k] = fx_mul(hrow[i], X[k]) + (fx_mul(q, Y[k]) >> min(down, 63)) + (flip ? P[k][i] : P[i][k]);
           }
-          store_row(blk + 4 * i, K[0], K[1], K[2], fx_mul(fU, hrow[i]));
+          store_row(blk + 4 * i, K[0], K[1], K[2], fx_mul1(fU, hrow[i]));
         }
         const int xp = bP + ecol - 2102;
         long long K3[3];
@@ -1130,7 +1161,7 @@ __global__ void __launch_bounds__(ELEMS * SPLIT, 384 / (ELEMS * SPLIT)) k_elem_f
           fx_acc(K3[k], xp, (flip ? -D[k] : D[k]) - T3[k], xs);
         }
         store_row(blk + 12, K3[0], K3[1], K3[2], pp);
-        store_exps(row, col, x, bU + erow - 2102, max(xp, xs), xpp);
+        store_exps(row, col, x, bU + erow - 2103, max(xp, xs), xpp);
       };
       block(r, c, hr, hc, er, ec, false);
       block(c, r, hc, hr, ec, er, true);
@@ -1473,6 +1504,68 @@ struct RowSum {
 // against 268 us for the FP64 gathers, which the shorter element phase and the
 // single launch come on top of; with the lists fetched where they are used the
 // kernel took 257 us, with the lists of two passes in registers 283 us.
+// A row with an element whose record is in FP64 is summed again in FP64
+// (384,000 elements, all of them such: 1.34 ms a neo-Hookean chain, J2 1.53;
+// 0.1% of them: 0.56 -> 0.62 and 0.62 -> 0.69).
+
+// The 4x4 block whose row r a lane of the quad holds, transposed.
+template <bool ADJ>
+__device__ __forceinline__ void transpose_quad(double (&d)[4], int r) {
+  if (!ADJ) return;
+  const unsigned full = 0xffffffffu;
+  const bool hi = (r & 2) != 0, odd = (r & 1) != 0;
+  const double s0 = __shfl_xor_sync(full, hi ? d[0] : d[2], 2), s1 = __shfl_xor_sync(full, hi ? d[1] : d[3], 2);
+  const double a0 = hi ? s0 : d[0], a1 = hi ? s1 : d[1], a2 = hi ? d[2] : s0, a3 = hi ? d[3] : s1;
+  const double t0 = __shfl_xor_sync(full, odd ? a0 : a1, 1), t1 = __shfl_xor_sync(full, odd ? a2 : a3, 1);
+  d[0] = odd ? t0 : a0; d[1] = odd ? a1 : t0; d[2] = odd ? t1 : a2; d[3] = odd ? a3 : t1;
+}
+// Row [k0, k0 + nk) of the matrix by one warp, diagonal block kd: the terms in
+// list order, the diagonal's u columns as negated sums of the row's blocks.
+template <bool ADJ>
+__device__ __noinline__ void gather_row_fp64(int k0, int nk, int kd, const int* btr, const int* bptr, const int* blist,
+                                             const long long* rec, double* A) {
+  const int lane = threadIdx.x & 31, q = lane >> 2, r = lane & 3;
+  const unsigned full = 0xffffffffu;
+  auto value = [](long long v, int e) { return e == kFxFloat ? __longlong_as_double(v) : fx_double(v, e); };
+  auto exps = [&](const long long* p, int l) { return reinterpret_cast<const int*>(p + kRecExp + (l & 15))[r == 3 ? 1 : 0]; };
+  double u[3] = {0.0, 0.0, 0.0};
+  for (int i0 = 0; i0 < nk - 1; i0 += 8) {
+    const bool live = i0 + q < nk - 1;
+    const int k = k0 + i0 + q + (i0 + q >= kd ? 1 : 0);
+    double d[4] = {0.0, 0.0, 0.0, 0.0};
+    if (live) {
+      for (int c = bptr[k]; c < bptr[k + 1]; ++c) {
+        const int l = blist[c];
+        const long long* p = rec + (size_t)(l >> 4) * kRecord;
+        const int e = exps(p, l);
+        const long long* v = p + kRecOff + 16 * off_index((l >> 2) & 3, l & 3) + 4 * r;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) d[j] += value(v[j], j < 3 ? (short)e : e >> 16);
+      }
+#pragma unroll
+      for (int j = 0; j < 3; ++j) u[j] += d[j];
+    }
+    transpose_quad<ADJ>(d, r);
+    if (live) st4(A + 16ll * (ADJ ? btr[k] : k) + 4 * r, d[0], d[1], d[2], d[3]);
+  }
+  double d[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int i = bptr[k0 + kd] + q; i < bptr[k0 + kd + 1]; i += 8) {
+    const int l = blist[i];
+    const long long* p = rec + (size_t)(l >> 4) * kRecord;
+    d[3] += value(p[kRecDiag + 4 * (l & 3) + r], exps(p, l) >> 16);
+  }
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {
+    d[3] += __shfl_xor_sync(full, d[3], o);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) u[j] += __shfl_xor_sync(full, u[j], o);
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) d[j] = -u[j];
+  transpose_quad<ADJ>(d, r);
+  if (q == 0) st4(A + 16ll * (k0 + kd) + 4 * r, d[0], d[1], d[2], d[3]);
+}
+
 constexpr int kRowTerms = 192;  // list entries of a row kept in shared memory (96 on the Kuhn grid)
 template <bool ADJ>
 __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, const int* __restrict__ brow_ptr,
@@ -1508,15 +1601,6 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
   }
   const int lane = threadIdx.x & 31, q = lane >> 2, r = lane & 3;
   const unsigned full = 0xffffffffu;
-  // the 4x4 block whose row r a lane of the quad holds, transposed
-  auto transpose = [&](double (&d)[4]) {
-    const bool hi = (r & 2) != 0, odd = (r & 1) != 0;
-    const double s0 = __shfl_xor_sync(full, hi ? d[0] : d[2], 2), s1 = __shfl_xor_sync(full, hi ? d[1] : d[3], 2);
-    const double a0 = hi ? s0 : d[0], a1 = hi ? s1 : d[1], a2 = hi ? d[2] : s0, a3 = hi ? d[3] : s1;
-    const double t0 = __shfl_xor_sync(full, odd ? a0 : a1, 1), t1 = __shfl_xor_sync(full, odd ? a2 : a3, 1);
-    d[0] = odd ? t0 : a0; d[1] = odd ? a1 : t0; d[2] = odd ? t1 : a2; d[3] = odd ? a3 : t1;
-  };
-  const double nan = __longlong_as_double(0x7ff8000000000000ll);
   // no load below can be moved ahead of this: each is under the loop's condition
   asm volatile("griddepcontrol.wait;" ::: "memory");
   constexpr int kNone = -32768;  // exponent of no term: every shift takes it to zero
@@ -1601,13 +1685,12 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
           else add(std::integral_constant<int, 2>(), terms + c, c1 - c, extra, acc, x0, x3);
         }
         row.add(acc, x0);
-        const bool bad0 = x0 >= kFxBad, bad3 = x3 >= kFxBad;
-        d[0] = bad0 ? nan : fx_double(acc[0], x0);
-        d[1] = bad0 ? nan : fx_double(acc[1], x0);
-        d[2] = bad0 ? nan : fx_double(acc[2], x0);
-        d[3] = bad3 ? nan : fx_double(acc[3], x3);
+        d[0] = fx_double(acc[0], x0);
+        d[1] = fx_double(acc[1], x0);
+        d[2] = fx_double(acc[2], x0);
+        d[3] = fx_double(acc[3], x3);
       }
-      if (ADJ) transpose(d);
+      transpose_quad<ADJ>(d, r);
       if (live) st4(A + 16ll * (ADJ ? __ldg(btr + k0 + k) : k0 + k) + 4 * r, d[0], d[1], d[2], d[3]);
     }
     // column 3 of the diagonal block: the terms of block kd are the node's elements
@@ -1635,6 +1718,11 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
       rx = max(rx, __shfl_xor_sync(full, rx, o));
       ex = max(ex, __shfl_xor_sync(full, ex, o));
     }
+    // an element in FP64 is among the terms of the diagonal block, as of the others
+    if (ex >= kFxFloat) {
+      gather_row_fp64<ADJ>(k0, nk, kd, btr, bptr, blist, rec, A);
+      continue;
+    }
     dacc >>= fx_shift(ex - dx);
     row.raise(rx);
     // the row sums as 64 bits, shifted so far that eight of them cannot overflow
@@ -1657,11 +1745,10 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
       for (int k = 0; k < 3; ++k) t[k] += __shfl_xor_sync(full, t[k], o);
     }
     double d[4];
-    const bool badr = rx >= kFxBad, badd = ex >= kFxBad;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) d[k] = badr ? nan : fx_double(-t[k], rx + sh);
-    d[3] = badd ? nan : fx_double(dacc, ex);
-    if (ADJ) transpose(d);
+    for (int k = 0; k < 3; ++k) d[k] = fx_double(-t[k], rx + sh);
+    d[3] = fx_double(dacc, ex);
+    transpose_quad<ADJ>(d, r);
     if (q == 0) st4(A + 16ll * (k0 + kd) + 4 * r, d[0], d[1], d[2], d[3]);
   }
 }
@@ -1863,8 +1950,13 @@ double assemble(Mechanics& m, SolInfo* s, const Chain& c, const ErrorWeights* w,
     a.estride = c.jacobian ? 272 : 16;
     const size_t per_elem = sizeof(double) * (a.estride + ((c.jacobian && c.qoi != QOI_NONE) ? 16 : 0));
     chunk = (int)std::max<long long>(1, std::min<long long>(E, element_buffer_limit() / per_elem));
-    // fixed point and diagonal blocks from row sums: Jacobian chains that overwrite, in one pass
-    fix = scatter && c.jacobian && c.overwrite && chunk == E;
+    // Fixed point and diagonal blocks from row sums: Jacobian chains that overwrite,
+    // in one pass, unless the mesh has so many flat elements that their second
+    // evaluation, by whole warps, would cost more than it saves (384,000 elements,
+    // us: FP64 throughout 997 neo-Hookean, 1,114 J2; fixed point with no flat
+    // element 562 and 621, with 0.1% 625 and 695, with all of them 1,386 and 1,581;
+    // one in 64 puts one into four of ten warps).
+    fix = scatter && c.jacobian && c.overwrite && chunk == E && 64ll * d.flat_elems <= E;
     if (fix) {
       a.estride = kRecord;
       if (c.mode == MODE_ADJOINT) const_cast<Disc&>(d).block_transpose_map();

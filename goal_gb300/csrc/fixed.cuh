@@ -3,15 +3,17 @@
 //
 // On this part an FP64 instruction takes an SM's pipe 19 clocks per warp, a
 // 32 x 32 -> 64 bit multiply-add 1.2 and a 64-bit add 0.5 (measured), so a sum
-// of products of numbers that share a scale is cheaper in integers, and exact
-// to more bits. A quantity is S 2^x: S a signed 64-bit integer, x an exponent
-// shared by the quantities that are added.
+// of products of numbers that share a scale is cheaper in integers. A quantity is
+// S 2^x: S a signed 64-bit integer, x an exponent shared by the quantities that
+// are added.
 //
 // A factor has up to 62 bits and is held as two signed 32-bit limbs; a product
 // keeps the limbs' high and middle partial products, S = (f g) / 2^64 to
-// within a unit, with |S| <= 2^60 for 62-bit factors. So a sum of products is
-// off by some 2^-59 of the largest product that its group's scale admits,
-// against 2^-53 in FP64.
+// within a unit, with |S| <= 2^60 for 62-bit factors. So a sum is off by a few
+// units of 2^-59 of the largest product that the exponents of its factors admit.
+// That is less than FP64's error only where its largest term is within some 2^-5
+// of that bound, and says nothing about an entry far below the largest that
+// shares its exponent: the caller looks at both (k_elem_fix).
 #pragma once
 
 #include "common.cuh"
@@ -21,7 +23,12 @@ namespace goal {
 #ifdef __CUDACC__
 
 constexpr int kFxMinExp = 64;       // least biased exponent of a scale: smaller numbers count as zero
-constexpr int kFxBad = 0x7fff;      // exponent of a quantity that is not finite
+constexpr int kFxFloat = 0x7fff;    // in place of an exponent: the entries are FP64
+
+// Largest difference of the exponents of an element's gradients in x, y and z.
+// The entries of a block differ by its square, and one of 2^-10 of the largest
+// is held to some 49 bits, as good as in FP64 after its few roundings.
+constexpr int kFxSpread = 5;
 
 struct Fx {
   int hi, lo;  // value hi 2^32 + lo
@@ -30,6 +37,9 @@ struct Fx {
 // Biased exponent of |v| (0x7ff: infinite or not a number), in the running
 // maximum of the high words of a group.
 __device__ __forceinline__ int fx_high(double v) { return __double2hiint(v) & 0x7fffffff; }
+__device__ __forceinline__ int fx_spread(const int (&x)[3]) {
+  return max(x[0], max(x[1], x[2])) - min(x[0], min(x[1], x[2]));
+}
 __device__ __forceinline__ int fx_exp(int high) { return max(high >> 20, kFxMinExp); }
 
 // v / 2^x, rounded, for |v| < 2^(x + 62)
@@ -64,6 +74,11 @@ __device__ __forceinline__ long long fx_mul(const Fx& f, const Fx& g) {
   const long long m = fx_mad(f.lo, g.hi, fx_mad(f.hi, g.lo, 0x80000000ll));
   return fx_mad(f.hi, g.hi, m >> 32);
 }
+// f g / 2^63
+__device__ __forceinline__ long long fx_mul1(const Fx& f, const Fx& g) {
+  const long long m = fx_mad(f.lo, g.hi, fx_mad(f.hi, g.lo, 0x40000000ll));
+  return (fx_mad(f.hi, g.hi, 0) << 1) + (m >> 31);
+}
 
 // Sums of up to three products of 60-bit factors, with five bits more:
 // sum / 2^59. High parts in s, middle parts in m (at 2^32).
@@ -74,7 +89,8 @@ struct FxSum {
     m = fx_mad(a.hi, b.lo, m);
     m = fx_mad(a.lo, b.hi, m);
   }
-  __device__ __forceinline__ long long value5() const { return (s << 5) + (m >> 27); }
+  template <int B>
+  __device__ __forceinline__ long long value() const { return (s << B) + (m >> (32 - B)); }  // sum / 2^(64 - B)
   // with the product of the low limbs, where a difference of two large numbers follows
   __device__ __forceinline__ void add_low(const Fx& a, const Fx& b) { m += fx_mad(a.lo, b.lo, 0x80000000ll) >> 32; }
 };
