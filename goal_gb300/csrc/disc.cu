@@ -625,10 +625,13 @@ void Disc::csr_graph(int* row_ptr_h, int* col_idx_h) const {
 }
 
 void Disc::block_transpose_map() {
+  std::lock_guard<std::mutex> lock(btr_guard);
   if (btr.ptr) return;
-  btr.alloc(nnzb);
-  k_block_transpose<<<grid_for(num_nodes, 256), 256, 0, stream>>>(num_nodes, brow_ptr.ptr, bcol.ptr, btr.ptr);
+  DevBuf<int> map;
+  map.alloc(nnzb);
+  k_block_transpose<<<grid_for(num_nodes, 256), 256, 0, stream>>>(num_nodes, brow_ptr.ptr, bcol.ptr, map.ptr);
   GOAL_CHECK_LAUNCH();
+  btr = std::move(map);
 }
 
 void Disc::csr_graph_device() {

@@ -19,6 +19,7 @@
 
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -109,8 +110,10 @@ struct Disc {
   // built on the first request for device pointers
   DevBuf<int> csr_row_ptr, csr_col_idx;
   // btr[k]: index of block (m, n) for block k = (n, m); built by the first
-  // transposed (ADJOINT) assembly
+  // transposed (ADJOINT) assembly, of several threads' by the one that holds the
+  // guard: the map is launched on this stream before any of them sees it
   DevBuf<int> btr;
+  std::mutex btr_guard;
 
   void build();                // Disc::build_data: graph, colouring, geometry
   DiscView view() const;
