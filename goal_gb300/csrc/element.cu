@@ -319,6 +319,8 @@ __device__ __forceinline__ void eval_point(const ElemArgs& a, bool save, int s, 
 // -> 126, of 384k 663 -> 753, residual of 48k 51 -> 60).
 __device__ __forceinline__ void gather_may_start() { asm volatile("griddepcontrol.launch_dependents;"); }
 // The address that loads after the wait use, so that none can move ahead of it.
+// They are plain loads: the blocks are on the chip while the element phase writes,
+// and the read-only path is for what stays as it is for the whole kernel.
 template <typename T>
 __device__ __forceinline__ const T* wait_for_elements(const T* buffer) {
   asm volatile("griddepcontrol.wait;" : "+l"(buffer)::"memory");
@@ -1441,7 +1443,7 @@ __global__ void __launch_bounds__(256) k_gather_blocks_chunk(int count, const in
 // [lo, hi): the element slots the buffer holds (a chunk; the buffer's first
 // entry is slot lo); the one-pass gather has lo = 0, hi = E.
 __global__ void __launch_bounds__(256) k_gather_nodes(int N, const int* __restrict__ nptr,
-                                                      const int* __restrict__ nlist, const double* __restrict__ ebuf,
+                                                      const int* __restrict__ nlist, const double* ebuf,
                                                       int estride, double* __restrict__ out, int accumulate, int lo,
                                                       int hi) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < 4ll * N;
@@ -1453,7 +1455,7 @@ __global__ void __launch_bounds__(256) k_gather_nodes(int N, const int* __restri
     for (int c = c0; c < c1; ++c) {
       const int v = __ldg(nlist + c), e = v >> 2;
       if (e < lo || e >= hi) continue;
-      acc += __ldg(buf + (size_t)(e - lo) * estride + 4 * (v & 3) + q);
+      acc += buf[(size_t)(e - lo) * estride + 4 * (v & 3) + q];
     }
     out[t] = acc;
   }
@@ -1572,8 +1574,8 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
                                                      const int* __restrict__ diag, const int* __restrict__ btr,
                                                      const int* __restrict__ bptr, const int* __restrict__ blist,
                                                      const int* __restrict__ nptr, const int* __restrict__ nlist,
-                                                     const long long* __restrict__ rec, double* __restrict__ A,
-                                                     double* __restrict__ R, const double* __restrict__ dbuf,
+                                                     const long long* records, double* __restrict__ A,
+                                                     double* __restrict__ R, const double* dbuf,
                                                      double* __restrict__ dMdu) {
   if ((int)blockIdx.x >= row_blocks) {
     const long long vectors = 2;  // R, then dM/du
@@ -1583,7 +1585,7 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
       const long long i = second ? t - 4ll * N : t;
       const int n = (int)(i >> 2), q = (int)(i & 3);
       const int c0 = __ldg(nptr + n), c1 = __ldg(nptr + n + 1);
-      const double* src = wait_for_elements(second ? dbuf : reinterpret_cast<const double*>(rec));
+      const double* src = wait_for_elements(second ? dbuf : reinterpret_cast<const double*>(records));
       if (second && !dbuf) {  // no QoI: dM/du is cleared
         dMdu[i] = 0.0;
         continue;
@@ -1593,7 +1595,7 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
 #pragma unroll 4
       for (int c = c0; c < c1; ++c) {
         const int v = __ldg(nlist + c);
-        acc += __ldg(src + (size_t)(v >> 2) * stride + 4 * (v & 3) + q);
+        acc += src[(size_t)(v >> 2) * stride + 4 * (v & 3) + q];
       }
       (second ? dMdu : R)[i] = acc;
     }
@@ -1601,8 +1603,7 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
   }
   const int lane = threadIdx.x & 31, q = lane >> 2, r = lane & 3;
   const unsigned full = 0xffffffffu;
-  // no load below can be moved ahead of this: each is under the loop's condition
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const long long* rec = wait_for_elements(records);
   constexpr int kNone = -32768;  // exponent of no term: every shift takes it to zero
   __shared__ int lists[4][kRowTerms];
   int* mine = lists[threadIdx.x >> 5];
@@ -1619,7 +1620,7 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
       if (u < left) {
         const int l = w[u];
         const long long* p = rec + (size_t)(l >> 4) * kRecord;
-        const int e = __ldg(reinterpret_cast<const int*>(p + kRecExp + (l & 15)) + (r == 3 ? 1 : 0));
+        const int e = reinterpret_cast<const int*>(p + kRecExp + (l & 15))[r == 3 ? 1 : 0];
         v[u] = *reinterpret_cast<const longlong4_32a*>(p + kRecOff + 16 * off_index((l >> 2) & 3, l & 3) + 4 * r);
         e0[u] = (short)e + extra;
         e3[u] = (e >> 16) + extra;
@@ -1704,9 +1705,9 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
       for (int i = c + q; i < c1; i += 8) {
         const int l = terms[i];
         const long long* p = rec + (size_t)(l >> 4) * kRecord;
-        const int e = (__ldg(reinterpret_cast<const int*>(p + kRecExp + (l & 15)) + (r == 3 ? 1 : 0)) >> 16) + extra;
+        const int e = (reinterpret_cast<const int*>(p + kRecExp + (l & 15))[r == 3 ? 1 : 0] >> 16) + extra;
         const int top = max(dx, e), sa = min(top - dx, 62), sv = min(top - e + extra, 62);
-        const long long v = __ldg(p + kRecDiag + 4 * (l & 3) + r);
+        const long long v = p[kRecDiag + 4 * (l & 3) + r];
         dacc = ((dacc + ((1ll << sa) >> 1)) >> sa) + ((v + ((1ll << sv) >> 1)) >> sv);
         dx = top;
       }
