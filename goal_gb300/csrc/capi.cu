@@ -7,6 +7,7 @@
 #include "../../include/goal_gb300.h"
 #include "capi_internal.cuh"
 #include "driver.cuh"
+#include "grid_barrier.cuh"
 #include "mpnn.cuh"
 #include "size_field.cuh"
 
@@ -15,6 +16,13 @@ namespace goal {
 std::atomic<long long> g_launches{0};
 static thread_local std::string t_last_error;
 void set_last_error(const std::string& msg) { t_last_error = msg; }
+
+static std::atomic<int> g_wait_limit{0};
+int wait_limit() {
+  const int set = g_wait_limit.load();
+  return set > 0 ? set : kWaitLimit;
+}
+void set_wait_limit(int looks) { g_wait_limit.store(looks); }
 
 namespace {
 
@@ -203,6 +211,13 @@ int goal_set_element_buffer_limit(long long bytes) {
   GOAL_API_BEGIN
   GOAL_ARG(bytes >= 0, "goal_set_element_buffer_limit: negative size");
   goal::set_element_buffer_limit(bytes);
+  GOAL_API_END
+}
+
+int goal_set_wait_limit(int looks) {
+  GOAL_API_BEGIN
+  GOAL_ARG(looks >= 0, "goal_set_wait_limit: negative limit");
+  goal::set_wait_limit(looks);
   GOAL_API_END
 }
 

@@ -146,6 +146,7 @@ struct ColorState {
   unsigned* size;   // ready elements of three successive rounds, in turn
   unsigned* count;  // barrier
   int* info;        // too many colours, rounds, a wait ran out
+  int limit;        // of a wait
 };
 constexpr int kColorThreads = 1024;
 __global__ void __launch_bounds__(kColorThreads, 1) k_color(int E, const int* __restrict__ tets,
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(kColorThreads, 1) k_color(int E, const int* __
   auto barrier = [&]() {
     __syncthreads();
     target += gridDim.x;
-    if (threadIdx.x == 0) ok = grid_meet(c.count, target) ? 1 : 0;
+    if (threadIdx.x == 0) ok = grid_meet(c.count, target, c.limit) ? 1 : 0;
     __syncthreads();
     return ok != 0;
   };
@@ -459,7 +460,7 @@ void Disc::build() {
     GOAL_CUDA(cudaGetDevice(&dev));
     GOAL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     unsigned* u = reinterpret_cast<unsigned*>(ctl);
-    ColorState cs{ca, wait, ready, u, u + 3, ctl + 4};
+    ColorState cs{ca, wait, ready, u, u + 3, ctl + 4, wait_limit()};
     int elems = E;
     void* args[] = {&elems, &tets_o, &ne_ptr, &ne_list, &cs};
     const int blocks = std::min(sms, (E + kColorThreads / 32 - 1) / (kColorThreads / 32));

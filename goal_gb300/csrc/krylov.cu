@@ -1239,6 +1239,7 @@ void launch_coop(const CoopPlan& p, CoopArgs<T, TA, TV> a, int nnzb, cudaStream_
   else if (smem + basis <= most / 2) smem += basis;
   a.chunk = p.chunk;
   a.smem_bytes = (int)std::min(smem, most);
+  a.limit = wait_limit();
   const void* kernel = (const void*)k_gmres_coop<T, TA, TV>;
   GOAL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem));
   void* args[] = {&a};

@@ -46,6 +46,7 @@ struct CoopArgs {
   GState* st;              // outer state (inner solve), or the state of this cycle
   int inner;
   int smem_bytes;
+  int limit;               // of a wait
 };
 
 __device__ __forceinline__ void coop_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kCoopThreads) : "memory"); }
@@ -64,11 +65,12 @@ struct CoopSync {
   unsigned* count;  // arrivals since the kernel began (cleared by the last CTA to leave)
   unsigned target;
   int* ok;          // shared
+  int limit;
 };
 
 // Warp 0 of every CTA, after a block barrier.
 __device__ __forceinline__ void coop_meet(CoopSync& s) {
-  if (threadIdx.x == 0) *s.ok = grid_meet(s.count, s.target) ? 1 : 0;
+  if (threadIdx.x == 0) *s.ok = grid_meet(s.count, s.target, s.limit) ? 1 : 0;
   __syncwarp();
 }
 
@@ -505,8 +507,13 @@ __global__ void __launch_bounds__(kCoopThreads + 32, 1) k_gmres_coop(const CoopA
   __shared__ GivensShared<T> gs;
   __shared__ int ok;
   __shared__ T newscale;
-  if (a.inner && a.st->done) return;  // the outer cycle is over: every CTA leaves
+  __shared__ int over;
   const int tid = threadIdx.x;
+  // The outer cycle is over: every CTA leaves. One thread looks, as a CTA whose
+  // wait ran out says so in the same place, and the barriers count all threads.
+  if (tid == 0) over = a.inner && *(volatile const int*)&a.st->done;
+  __syncthreads();
+  if (over) return;
   const int n0 = blockIdx.x * a.chunk, n1 = min(a.N, n0 + a.chunk);
   const int nodes = max(0, n1 - n0), rows = 4 * nodes, cap = 4 * a.chunk;
   const long long n = 4ll * a.N;
@@ -544,7 +551,7 @@ __global__ void __launch_bounds__(kCoopThreads + 32, 1) k_gmres_coop(const CoopA
       givens_warp<T>(&gs, gcol, grot, glow, gcs, gsn, gg, gdi, a.H, a.m + 1, a.y, a.tol_abs, a.inner ? nullptr : a.st);
     return;
   }
-  CoopSync sync{a.ctl + 2, 0u, &ok};
+  CoopSync sync{a.ctl + 2, 0u, &ok, a.limit};
   const T* Dinv = a.Dinv + 16ll * n0;
   const T* Bc = a.Bc ? a.Bc + 16ll * n0 : nullptr;
   auto stage_blocks = [&](const T* src) -> const T* {
@@ -644,15 +651,25 @@ __global__ void __launch_bounds__(kCoopThreads + 32, 1) k_gmres_coop(const CoopA
   };
   const int rows32 = (rows + 31) & ~31, ldp = a.m + 1;
 
+  // The column that the Givens warp has, if any, has to be back before the next
+  // arrival at its barrier, and after its last one it waits no more.
+  bool handed = false;
+  auto collect = [&]() {
+    givens_sync(kBarRotated);
+    handed = false;
+  };
   auto failed = [&]() {
     if (tid == 0) {
       a.st->pad = 1;
       a.st->done = 1;
     }
     if (blockIdx.x == 0) {
-      if (tid == 0) gs.quit = 1;
-      coop_bar();
-      givens_arrive(kBarColumn);
+      if (handed) collect();
+      if (!gs.done) {
+        if (tid == 0) gs.quit = 1;
+        coop_bar();
+        givens_arrive(kBarColumn);
+      }
     }
   };
 
@@ -720,7 +737,7 @@ __global__ void __launch_bounds__(kCoopThreads + 32, 1) k_gmres_coop(const CoopA
     // longest time to answer
     auto column_done = [&]() {
       if (blockIdx.x == 0 && cols > 0) {
-        givens_sync(kBarRotated);
+        collect();
         if (tid == 0) {
           a.ctl[0] = (unsigned)gs.done;
           a.ctl[1] = (unsigned)cols;
@@ -768,10 +785,11 @@ __global__ void __launch_bounds__(kCoopThreads + 32, 1) k_gmres_coop(const CoopA
         gs.last = live ? 0 : 1;
       }
       givens_arrive(kBarColumn);
+      handed = true;
     }
     if (!live) {
       if (blockIdx.x == 0) {
-        givens_sync(kBarRotated);
+        collect();
         if (tid == 0) a.ctl[1] = (unsigned)cols;
       }
       if (!grid_sync(sync)) { failed(); return; }

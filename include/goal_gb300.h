@@ -288,6 +288,12 @@ int goal_assemble(goal_mechanics m, goal_sol_info s, const goal_chain* chain, do
  * accumulating pass, so the results are the same bits as its. 0 (default) = a quarter of the
  * device's memory. Process-wide. */
 int goal_set_element_buffer_limit(long long bytes);
+/* No counterpart in the reference. For tests: how often a block of the kernels
+ * with barriers among all their blocks (the solver's persistent cycle, the
+ * colouring) looks at a barrier before it gives up. The call then returns
+ * GOAL_ERR_SOLVER or GOAL_ERR_STATE, and the next one starts afresh. 0 (default) =
+ * 4,194,304 looks, more than a second. Process-wide. */
+int goal_set_wait_limit(int looks);
 /* No counterpart in the reference. Device time of goal_assemble's two phases,
  * measured with CUDA events on the discretization's stream: enable != 0 clears
  * the sums and starts measuring, 0 stops. ms[0] = element kernel(s), ms[1] =
