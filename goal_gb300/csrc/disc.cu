@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <chrono>
 
+#include "coop_plan.h"
 #include "disc.cuh"
 #include "fixed.cuh"
 #include "grid_barrier.cuh"
@@ -456,15 +457,16 @@ void Disc::build() {
   int* ctl = tmp.take(8);
   GOAL_CUDA(cudaMemsetAsync(ctl, 0, sizeof(int) * 8, s));
   {
-    int dev = 0, sms = 0;
-    GOAL_CUDA(cudaGetDevice(&dev));
-    GOAL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const CoopDevice& dev = coop_device();
     unsigned* u = reinterpret_cast<unsigned*>(ctl);
     ColorState cs{ca, wait, ready, u, u + 3, ctl + 4, wait_limit()};
     int elems = E;
     void* args[] = {&elems, &tets_o, &ne_ptr, &ne_list, &cs};
-    const int blocks = std::min(sms, (E + kColorThreads / 32 - 1) / (kColorThreads / 32));
-    GOAL_CUDA(cudaLaunchCooperativeKernel((const void*)k_color, dim3(blocks), dim3(kColorThreads), args, 0, s));
+    const int blocks = std::min(dev.sms, (E + kColorThreads / 32 - 1) / (kColorThreads / 32));
+    if (dev.launches)
+      GOAL_CUDA(cudaLaunchCooperativeKernel((const void*)k_color, dim3(blocks), dim3(kColorThreads), args, 0, s));
+    else  // one block waits for no other
+      GOAL_CUDA(cudaLaunchKernel((const void*)k_color, dim3(1), dim3(kColorThreads), args, 0, s));
     GOAL_CHECK_LAUNCH();
     int h[8];
     GOAL_CUDA(cudaMemcpyAsync(h, ctl, sizeof(h), cudaMemcpyDeviceToHost, s));

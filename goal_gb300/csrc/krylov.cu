@@ -7,6 +7,7 @@
 #include <chrono>
 #include <cmath>
 
+#include "coop_plan.h"
 #include "grid_barrier.cuh"
 #include "krylov.cuh"
 
@@ -1167,17 +1168,6 @@ struct StepGraph {
 };
 }  // namespace
 
-namespace {
-
-// How a persistent cycle (k_gmres_coop) of N nodes is laid out: nodes per CTA
-// and CTAs, one CTA per SM at most.
-struct CoopPlan {
-  int chunk = 0, grid = 0;
-};
-
-struct CoopDevice {
-  int sms = 0, smem = 0;
-};
 const CoopDevice& coop_device() {
   constexpr int kDevs = 64;
   static CoopDevice known[kDevs];
@@ -1192,42 +1182,21 @@ const CoopDevice& coop_device() {
     GOAL_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     GOAL_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     GOAL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    GOAL_REQUIRE(coop, GOAL_ERR_CUDA, "cooperative launches are not available");
+    d.launches = coop != 0;
     d.smem = optin - 512;  // the kernel's static shared memory stays below this
     d.sms = sms;
   }
   return d;
 }
 
-// The persistent cycle wins while an Arnoldi step is bound by its launches and
-// its few blocks; far enough up, the separate kernels with their more threads in
-// flight on the matrix and basis streams are faster, the earlier the more of a
-// step the products are. Whole solves to 1e-12, ms, kernels -> persistent:
-// binary16 inner 5k nodes 28.0 -> 11.3, 36k 58 -> 28, 59k 72.7 -> 44.4, 185k 230
-// -> 181, 275k 327 -> 303, 389k 520 -> 512, 531k 710 -> 781; with the second
-// sweep 149k 138 -> 109, 185k 182 -> 184, 227k 220 -> 234; binary32 133k 253 ->
-// 165, 227k 496 -> 329; FP64 inner 69k 318 -> 212, 133k 544 -> 469; FP64 343
-// 26.5 -> 3.9, 36k 1717 -> 828, 69k 5090 -> 3230 (not measured further up).
-constexpr int kCoopMinNodes = 8;  // of a CTA: a warp of rows
-constexpr int kCoopNodesPerSm = 2300, kCoopNodesPerSmSweep2 = 1150, kCoopNodesPerSmFp64 = 900;
-
-bool coop_plan(int N, bool fp64, bool sweep2, CoopPlan& p) {
-  const CoopDevice& d = coop_device();
-  const int per_sm = fp64 ? kCoopNodesPerSmFp64 : sweep2 ? kCoopNodesPerSmSweep2 : kCoopNodesPerSm;
-  if (N > per_sm * d.sms) return false;
-  p.chunk = std::max(kCoopMinNodes, (N + 8 * d.sms - 1) / (8 * d.sms) * 8);
-  p.grid = (N + p.chunk - 1) / p.chunk;
-  return true;
-}
+namespace {
 
 template <typename T, typename TA, typename TV>
 void launch_coop(const CoopPlan& p, CoopArgs<T, TA, TV> a, int nnzb, cudaStream_t s) {
   const CoopDevice& d = coop_device();
   const size_t cap = 4 * (size_t)p.chunk, most = (size_t)d.smem;
-  auto pad = [](size_t bytes) { return (bytes + 31) / 32 * 32; };  // as the kernel lays them out
-  // w, t, h, coefficients, scales, rotations, the reduction buffer, row pointers
-  const size_t fixed = (a.Bc ? 2 : 1) * pad(sizeof(T) * cap) + 11 * pad(sizeof(T) * (a.m + 2)) +
-                       pad(sizeof(T) * kCoopRed) + pad(sizeof(int) * (p.chunk + 1));
+  auto pad = coop_pad;
+  const size_t fixed = coop_fixed_bytes(p.chunk, a.m, sizeof(T), a.Bc != nullptr);
   GOAL_REQUIRE(fixed <= most, GOAL_ERR_CAPACITY, "persistent cycle: rows per CTA exceed shared memory");
   const size_t pitch = cap + (std::is_same<T, double>::value ? 1 : 32);
   const size_t blocks = (a.Bc ? 2 : 1) * pad(sizeof(T) * 4 * cap), basis = pad(sizeof(TV) * pitch * (a.m + 1));
@@ -1308,7 +1277,7 @@ void issue_inner(const BsrView& A, long long n, int mi, bool sweep2, GState* st,
   const int nbx = vec_grid(n);
   cudaStream_t s = K.stream;
   CoopPlan plan;
-  if (coop_plan(N, std::is_same<T, double>::value, sweep2, plan)) {
+  if (coop_plan(coop_device(), N, std::is_same<T, double>::value, sweep2, plan)) {
     CoopArgs<T, TA, TV> a{};
     a.N = N;
     a.m = mi;
@@ -1449,7 +1418,7 @@ SolveStats fgmres(const BsrView& A, const double* vals, const double* b, double*
   const int batch = mixed ? 1 : 4;
 
   CoopPlan plan;
-  const bool coop = !mixed && coop_plan(N, true, sweep2, plan);
+  const bool coop = !mixed && coop_plan(coop_device(), N, true, sweep2, plan);
   while (beta > tol_abs && out.iters < p.max_iters) {
     const int steps = std::min(m, p.max_iters - out.iters);
     int done_steps = 0;

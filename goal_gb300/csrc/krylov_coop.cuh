@@ -18,9 +18,6 @@
 //
 // Included by krylov.cu inside its anonymous namespace.
 
-constexpr int kCoopThreads = 512;            // worker threads of a CTA
-constexpr int kCoopWarps = kCoopThreads / 32;
-
 template <typename T, typename TA, typename TV>
 struct CoopArgs {
   int N;                   // nodes
@@ -143,8 +140,6 @@ template <typename T>
 __device__ __forceinline__ void ld_w(const T* p, T (&x)[4]) { Vec4<T>::load(p, x[0], x[1], x[2], x[3]); }
 template <typename T>
 __device__ __forceinline__ void ld_w(const T* p, T (&x)[1]) { x[0] = *p; }
-
-constexpr int kCoopRed = 32 * kCoopWarps;  // entries of the block-level reduction buffer
 
 // This CTA's partial sums of w . V_c for c < ncols, and of w . w as column
 // ncols if `self`, to part[CTA][column]. Two mappings:
