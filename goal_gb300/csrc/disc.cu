@@ -377,6 +377,23 @@ void sort_pairs(const Scratch& tmp, const int* kin, int* kout, const int* vin, i
   GOAL_CHECK_LAUNCH();
 }
 
+// The incidences of a side set as (node << 32) + incidence, by node and in side
+// order within a node: a radix sort, whose time is the set's own whatever the
+// mesh has of nodes.
+std::vector<uint64_t> sorted_incidences(const std::vector<int>& tris) {
+  std::vector<uint64_t> v(tris.size()), t(tris.size());
+  for (size_t k = 0; k < v.size(); ++k) v[k] = (uint64_t)(uint32_t)tris[k] << 32 | k;
+  for (int shift = 32; shift < 64; shift += 11) {
+    size_t at[2049] = {0};
+    for (uint64_t x : v) at[(x >> shift & 2047) + 1]++;
+    if (std::find(at + 1, at + 2049, v.size()) != at + 2049) continue;  // the same digit everywhere
+    for (int d = 0; d < 2048; ++d) at[d + 1] += at[d];
+    for (uint64_t x : v) t[at[x >> shift & 2047]++] = x;
+    v.swap(t);
+  }
+  return v;
+}
+
 int bits_for(int n) {
   int b = 1;
   while ((1ll << b) <= (long long)n) ++b;
@@ -558,17 +575,15 @@ void Disc::build() {
     SideSet& ss = *kv.second;
     int S = (int)ss.tris.size() / 3;
     ss.dtris.upload(ss.tris.data(), ss.tris.size(), s);
-    // incidences by node, in side order within a node
-    std::vector<int> start(N + 1, 0), nodes, ptr, inc(3 * (size_t)S);
-    for (int k = 0; k < 3 * S; ++k) start[ss.tris[k] + 1]++;
-    for (int n = 0; n < N; ++n) {
-      if (start[n + 1]) {
-        nodes.push_back(n);
-        ptr.push_back(start[n]);
+    std::vector<int> nodes, ptr, inc;
+    const std::vector<uint64_t> by_node = sorted_incidences(ss.tris);
+    for (size_t k = 0; k < by_node.size(); ++k) {
+      if (k == 0 || by_node[k] >> 32 != by_node[k - 1] >> 32) {
+        nodes.push_back((int)(uint32_t)(by_node[k] >> 32));
+        ptr.push_back((int)k);
       }
-      start[n + 1] += start[n];
+      inc.push_back((int)(uint32_t)by_node[k]);
     }
-    for (int k = 0; k < 3 * S; ++k) inc[start[ss.tris[k]]++] = k;
     ptr.push_back(3 * S);
     ss.nodes_h = nodes;
     ss.nodes.upload(nodes.data(), nodes.size(), s);
