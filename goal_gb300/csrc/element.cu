@@ -411,12 +411,12 @@ __device__ __forceinline__ void elem_fp64(const ElemArgs& a, bool save, int s) {
     if constexpr (!JAC && !ERR) {
       // A residual alone, which the FP64 pipe bounds (all of its time): V J sigma
       // F^-T = V sigma cof F, in the stabilization v . h_a with the cofactors on
-      // one side, and the last node from the others, as the gradients sum to
-      // zero: 102 FP64 instructions against 118 from h_a and J sigma, to the same
-      // error. (V gamma alpha (F C - Ic/3 F^-T) + p cof F would be 15 fewer, but
-      // the difference loses digits: error 1.3e-13 against 7e-14.) 384,000
-      // elements, J2, with the point's own 22 fewer: 257 us -> 234, neo-Hookean
-      // 194 -> 180.
+      // one side: 102 FP64 instructions against 118 from h_a and J sigma, to the
+      // same error. (V gamma alpha (F C - Ic/3 F^-T) + p cof F would be 15 fewer,
+      // but the difference loses digits: error 1.3e-13 against 7e-14. The last
+      // node's row as the negated sum of the others', whose digits it would have,
+      // gains nothing.) A chain of 384,000 elements, J2, with the point's own 22
+      // instructions fewer: 292 us -> 257.
       const double rp0 = ((pval * inv_kappa) - dUdJ) * 0.25 * V;
       double P[3][3], z[3] = {0.0, 0.0, 0.0};
 #pragma unroll
@@ -434,16 +434,11 @@ __device__ __forceinline__ void elem_fp64(const ElemArgs& a, bool save, int s) {
         for (int k = 0; k < 3; ++k) z[k] = pt.cof[0][k] * cg[0] + pt.cof[1][k] * cg[1] + pt.cof[2][k] * cg[2];
       }
 #pragma unroll
-      for (int n = 0; n < 3; ++n) {
+      for (int n = 0; n < 4; ++n) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) Ru[n][i] = fma(P[i][0], G[n][0], fma(P[i][1], G[n][1], P[i][2] * G[n][2]));
-        Rp[n] = fma(z[0], G[n][0], fma(z[1], G[n][1], z[2] * G[n][2]));
+        Rp[n] = fma(z[0], G[n][0], fma(z[1], G[n][1], fma(z[2], G[n][2], rp0)));
       }
-#pragma unroll
-      for (int i = 0; i < 3; ++i) Ru[3][i] = -((Ru[0][i] + Ru[1][i]) + Ru[2][i]);
-      Rp[3] = rp0 - ((Rp[0] + Rp[1]) + Rp[2]);
-#pragma unroll
-      for (int n = 0; n < 3; ++n) Rp[n] += rp0;
     } else if constexpr (!ERR) {
       double TV[3][3];  // V J sigma
 #pragma unroll
