@@ -62,3 +62,32 @@ def test_first_adjoint_assemblies_on_one_disc(again):
     _together([k[2] for k in kept])
     for (m, s, _), A in zip(kept, alone):
         assert np.array_equal(s.dRdu_csr(), A)
+
+
+def _program(n, seed, precision):
+    """A discretization, an assembly and a solve of its own, as one thread's program."""
+    mesh = kuhn_cube(n, jitter=0.2, seed=seed)
+    d = api.Disc(mesh)
+    m = api.Mechanics(d, api.J2, [ROW])
+    U = _state(mesh, seed)
+    U[:, 0] += 0.002 * mesh.coords[:, 0]
+    m.set_solution(U)
+    s = api.SolInfo(d)
+    api.assemble(m, s, api.PRIMAL, jacobian=True, save_states=True)
+    bcs = api.Bcs(d, [(0, "xmin", "0.0"), (1, "xmin", "0.0"), (2, "xmin", "0.0"), (0, "xmax", "0.002*t")], [])
+    api.set_jac_dbcs(m, s, bcs, 1.0)
+    x, st = api.solve(s, -s.R, params=api.solve_params(krylov_size=60, max_iters=20000, tolerance=1e-10,
+                                                       precision=precision, inner_iters=30))
+    assert st["converged"]
+    return d.colors(), s.dRdu_csr(), x
+
+
+@pytest.mark.parametrize("again", range(3))
+def test_programs_side_by_side(again):
+    """Colourings and persistent cycles, which take the whole chip each, on the
+    streams of four threads."""
+    jobs = [lambda n=n, p=p, k=k: _program(n, 10 * again + k, p)
+            for k, (n, p) in enumerate([(12, api.MIXED), (9, api.FP64), (12, api.MIXED_F32), (10, api.NESTED_F64)])]
+    alone = [j() for j in jobs]
+    for a, b in zip(alone, _together(jobs)):
+        assert all(np.array_equal(x, y) for x, y in zip(a, b))
