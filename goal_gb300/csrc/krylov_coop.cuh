@@ -790,7 +790,10 @@ __global__ void __launch_bounds__(kCoopThreads + 32, 1) k_gmres_coop(const CoopA
       if (!grid_sync(sync)) { failed(); return; }
       break;
     }
-    if (norm * s > T(8) || norm * s < T(0.125)) {  // the estimate lost its digits: store the column again
+    // Where the estimate lost its digits the column is stored again: it is to have
+    // unit norm at least, as a normalized one has, or binary16 would hold its small
+    // entries to fewer bits.
+    if (norm * s > T(8) || norm * s < T(1)) {
       s = pow2_rsqrt(norm * norm);
       publish(cols, s);
       if (!grid_sync(sync)) { failed(); return; }
