@@ -23,12 +23,17 @@ struct CoopPlan {
 // The persistent cycle wins while an Arnoldi step is bound by its launches and
 // its few blocks; far enough up, the separate kernels with their more threads in
 // flight on the matrix and basis streams are faster, the earlier the more of a
-// step the products are. Whole solves to 1e-12, ms, kernels -> persistent:
-// binary16 inner 5k nodes 28.0 -> 11.3, 36k 58 -> 28, 59k 72.7 -> 44.4, 185k 230
-// -> 181, 275k 327 -> 303, 389k 520 -> 512, 531k 710 -> 781; with the second
-// sweep 149k 138 -> 109, 185k 182 -> 184, 227k 220 -> 234; binary32 133k 253 ->
-// 165, 227k 496 -> 329; FP64 inner 69k 318 -> 212, 133k 544 -> 469; FP64 343
-// 26.5 -> 3.9, 36k 1717 -> 828, 69k 5090 -> 3230 (not measured further up).
+// step the products are. 100 columns in FP64, 3 x 60 inner ones else, ms, kernels ->
+// persistent, at nodes below and above each line:
+//   one sweep   binary16 301k 18.7 -> 16.8, 358k 22.9 -> 23.0, 405k 24.6 -> 25.3
+//               binary32 301k 31.9 -> 22.6, 358k 35.8 -> 33.7, 405k 38.3 -> 36.5
+//   two sweeps  binary16 149k 19.1 -> 15.5, 176k 22.0 -> 19.7, 227k 26.0 -> 28.9
+//               binary32 149k 26.9 -> 22.2, 176k 35.5 -> 26.8, 227k 40.4 -> 40.8
+//   FP64        one 104k 40.3 -> 30.3, 141k 42.6 -> 39.6, 227k 56.1 -> 62.3
+//               two 104k 48.3 -> 39.6, 141k 53.1 -> 52.0, 227k 72.5 -> 80.3
+//   FP64 inner  one 104k 32.5 -> 25.0, 141k 35.7 -> 32.6, 227k 48.5 -> 51.6
+//               two 104k 44.6 -> 40.1, 141k 52.0 -> 52.7, 227k 73.7 -> 80.4
+// and at 30k to 69k nodes 1.3 to 2 times faster throughout.
 constexpr int kCoopMinNodes = 8;  // of a CTA: a warp of rows
 constexpr int kCoopNodesPerSm = 2300, kCoopNodesPerSmSweep2 = 1150, kCoopNodesPerSmFp64 = 900;
 
