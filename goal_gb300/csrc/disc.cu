@@ -53,6 +53,11 @@ __global__ void k_node_adjacency(int N, const int* tets, const int* ne_ptr, cons
       if (lane == 0) atomicExch(err, 1);
       continue;
     }
+    if (m == 0) {  // a node of no element has its diagonal block, which diag[n] names
+      if (lane == 0 && bcol) bcol[brow_ptr[n]] = n;
+      if (lane == 0 && out_count) out_count[n] = 1;
+      continue;
+    }
     int cnt = 4 * m;
     int P = 32;
     while (P < cnt) P <<= 1;
