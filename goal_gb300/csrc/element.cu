@@ -319,8 +319,8 @@ __device__ __forceinline__ void eval_point(const ElemArgs& a, bool save, int s, 
 // -> 126, of 384k 663 -> 753, residual of 48k 51 -> 60).
 __device__ __forceinline__ void gather_may_start() { asm volatile("griddepcontrol.launch_dependents;"); }
 // The address that loads after the wait use, so that none can move ahead of it.
-// They are plain loads: the blocks are on the chip while the element phase writes,
-// and the read-only path is for what stays as it is for the whole kernel.
+// They are not read-only loads: the blocks are on the chip while the element phase
+// writes, and that path is for what stays as it is for the whole kernel.
 template <typename T>
 __device__ __forceinline__ const T* wait_for_elements(const T* buffer) {
   asm volatile("griddepcontrol.wait;" : "+l"(buffer)::"memory");
@@ -1505,6 +1505,17 @@ struct RowSum {
 // (384,000 elements, all of them such: 1.34 ms a neo-Hookean chain, J2 1.53;
 // 0.1% of them: 0.56 -> 0.62 and 0.62 -> 0.69).
 
+// Row of a record's block. Each is read once, and leaves L1 to the lists and
+// exponents (gather of 384,000 elements: 237 us through L1, 230 past it; exponents
+// past it too 229, but the chain of 384 elements 39.3 -> 40.0).
+__device__ __forceinline__ longlong4_32a ld_row(const long long* p) {
+  longlong4_32a v;
+  asm volatile("ld.global.L1::no_allocate.v4.s64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(v.x), "=l"(v.y), "=l"(v.z), "=l"(v.w)
+               : "l"(p));
+  return v;
+}
+
 // The 4x4 block whose row r a lane of the quad holds, transposed.
 template <bool ADJ>
 __device__ __forceinline__ void transpose_quad(double (&d)[4], int r) {
@@ -1616,7 +1627,7 @@ __global__ void __launch_bounds__(128, 8) k_gather_rows(int N, int row_blocks, c
         const int l = w[u];
         const long long* p = rec + (size_t)(l >> 4) * kRecord;
         const int e = reinterpret_cast<const int*>(p + kRecExp + (l & 15))[r == 3 ? 1 : 0];
-        v[u] = *reinterpret_cast<const longlong4_32a*>(p + kRecOff + 16 * off_index((l >> 2) & 3, l & 3) + 4 * r);
+        v[u] = ld_row(p + kRecOff + 16 * off_index((l >> 2) & 3, l & 3) + 4 * r);
         e0[u] = (short)e + extra;
         e3[u] = (e >> 16) + extra;
       }
