@@ -1,7 +1,11 @@
 // Element kernels: residual, hand-derived tangent, QoI and DWR error chain of
-// goal's stabilized mixed u-p mechanics on linear tets, one thread per element,
-// elements of one colour per launch (no two of them share a node, so the
-// scatter into the 4x4-block matrix needs no atomics and is deterministic).
+// goal's stabilized mixed u-p mechanics on linear tets. By default one launch
+// evaluates all elements into a buffer (a thread each: k_elem in FP64; k_elem_fix,
+// the tangent of an overwriting Jacobian chain in 64-bit fixed point, with up to
+// four threads to an element of a small mesh) and a second sums each matrix block
+// and nodal row over its elements. Coloured chains accumulate in place, elements
+// of one colour per launch (no two of them share a node). Neither needs atomics;
+// both are deterministic.
 //
 // Reference chain (one integration point, src/goal_assembly.cpp:65-88):
 //   Kinematics F = I + grad u, J = det F                   src/goal_kinematics.cpp:18-25
@@ -748,9 +752,9 @@ __device__ __noinline__ void record_fp64(const ElemArgs& a, int s) {
 // and the loops over nodes and pairs are not unrolled: unrolled, the kernel
 // was 12,800 instructions long and waited for instruction fetches 43% of the
 // time. J2 at 384,000 elements: 740 us in FP64 throughout, 1,208 unrolled, 498
-// with FP64 vectors m, q, n, X, Y, Z, now 422 (neo-Hookean 327). What bounds
-// it is latency at three warps per scheduler (registers and shared memory);
-// the FP64 pipe is 66% busy.
+// with FP64 vectors m, q, n, X, Y, Z, 422 with one exponent for all factors, now
+// 427 (neo-Hookean 327, 324). What bounds it is latency at three warps per
+// scheduler (registers and shared memory); the FP64 pipe is 65% busy.
 //
 // SPLIT threads in different warps share an element of a small mesh, where one
 // thread's chain of dependent instructions is all the time there is (36 us with
@@ -1497,7 +1501,7 @@ struct RowSum {
 // k_gather_nodes does (four threads per node, element order): R from the
 // records, and dM/du from dbuf, or zero without one.
 // The sums need no FP64 instruction but one conversion per matrix entry. At
-// 384,000 elements 231 us (3.9 TB/s; latency and the integer pipes, 47% busy)
+// 384,000 elements 230 us (4.1 TB/s; latency and the integer pipes, 47% busy)
 // against 268 us for the FP64 gathers, which the shorter element phase and the
 // single launch come on top of; with the lists fetched where they are used the
 // kernel took 257 us, with the lists of two passes in registers 283 us.
