@@ -576,6 +576,7 @@ void Disc::build() {
 
   // node sets / side sets to the device
   for (auto& kv : node_sets) kv.second->dev.upload(kv.second->host.data(), kv.second->host.size(), s);
+  std::vector<std::vector<int>> sent;  // until the copies are done
   for (auto& kv : side_sets) {
     SideSet& ss = *kv.second;
     int S = (int)ss.tris.size() / 3;
@@ -594,6 +595,7 @@ void Disc::build() {
     ss.nodes.upload(nodes.data(), nodes.size(), s);
     ss.inc_ptr.upload(ptr.data(), ptr.size(), s);
     ss.inc.upload(inc.data(), inc.size(), s);
+    for (auto* v : {&nodes, &ptr, &inc}) sent.push_back(std::move(*v));
   }
   phase(4);
   built = true;

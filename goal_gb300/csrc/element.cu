@@ -1810,6 +1810,7 @@ void Mechanics::init() {
   ticket.alloc(1);
   ticket.zero(disc->stream);
   results.alloc();
+  GOAL_CUDA(cudaStreamSynchronize(disc->stream));  // the material rows above leave with this call
 }
 
 void Mechanics::refresh_cpinv() {
