@@ -388,10 +388,12 @@ void sort_pairs(const Scratch& tmp, const int* kin, int* kout, const int* vin, i
 std::vector<uint64_t> sorted_incidences(const std::vector<int>& tris) {
   std::vector<uint64_t> v(tris.size()), t(tris.size());
   for (size_t k = 0; k < v.size(); ++k) v[k] = (uint64_t)(uint32_t)tris[k] << 32 | k;
+  uint64_t differ = 0;
+  for (uint64_t x : v) differ |= x ^ v[0];
   for (int shift = 32; shift < 64; shift += 11) {
-    size_t at[2049] = {0};
+    if (!(differ >> shift & 2047)) continue;
+    unsigned at[2049] = {0};
     for (uint64_t x : v) at[(x >> shift & 2047) + 1]++;
-    if (std::find(at + 1, at + 2049, v.size()) != at + 2049) continue;  // the same digit everywhere
     for (int d = 0; d < 2048; ++d) at[d + 1] += at[d];
     for (uint64_t x : v) t[at[x >> shift & 2047]++] = x;
     v.swap(t);
@@ -541,8 +543,7 @@ void Disc::build() {
   GOAL_CHECK_LAUNCH();
   color_ptr.resize(kMaxColors + 2);
   GOAL_CUDA(cudaMemcpyAsync(color_ptr.data(), cptr, sizeof(int) * (kMaxColors + 2), cudaMemcpyDeviceToHost, s));
-  GOAL_CUDA(cudaStreamSynchronize(s));
-  phase(2);
+  phase(2);  // waits for the stream
   flat_elems = color_ptr[kMaxColors + 1];
   // colours are numbered without gaps: the first one past the last colour starts at E
   num_colors = 0;
