@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 
 from goal_gb300 import api
-from goal_gb300.mesh import Mesh, kuhn_cube
+from goal_gb300.mesh import Mesh, kuhn_cube, orient_positive
 
 pytestmark = pytest.mark.gpu
 
@@ -212,6 +212,31 @@ def test_flat_elements_are_left_to_fp64(n, flat, mode):
 
 
 @pytest.mark.parametrize("mode", [api.PRIMAL, api.ADJOINT])
+@pytest.mark.parametrize("m", [3, 17, 33, 127])
+def test_long_rows_in_fp64(m, mode):
+    """A pinwheel of m tets around an edge, flattened by the state: rows with more
+    blocks than a warp has lanes and more terms than the gather keeps ahead."""
+    t = 2 * np.pi * np.arange(m) / m
+    ring = np.stack([np.cos(t), np.sin(t), 0.5 + 0.1 * np.sin(3 * t)], axis=1)
+    coords = np.concatenate([[[0.0, 0.0, 0.0], [0.0, 0.0, 1.0]], ring])
+    tets = orient_positive(coords, np.array([[0, 1, 2 + i, 2 + (i + 1) % m] for i in range(m)], np.int32))
+    mesh = Mesh(coords=coords, tets=tets, elem_set=np.zeros(m, np.int32), elem_set_names=["a"], node_sets={},
+                side_sets={})
+    U = _deformed(mesh, np.diag([1.0, 1.0, 1e-4]), 1e-8 / m)
+    d, s, z, _, _ = _both(mesh, api.NEOHOOKEAN, U, mode)
+    # the terms of each row, which cancel in some: a sum of up to m element blocks, each of some
+    # ten roundings, and on the diagonal the sum of the row
+    K = np.abs(_blocks(mesh, api.NEOHOOKEAN, U, None, None)).astype(float)
+    terms = np.zeros((d.num_nodes, 4))
+    for a in range(4):
+        np.add.at(terms, mesh.tets[:, a], K[:, a].sum((1, 3)) if mode == api.PRIMAL else K[:, :, a].sum((1, 2)))
+    off = np.abs(s.dRdu_csr() - z.dRdu_csr())
+    rp = d.graph()[0]
+    assert np.all(np.maximum.reduceat(off, rp[:-1]) <= (m + 16) * 2.0 ** -52 * terms.ravel())
+    assert np.array_equal(s.R, z.R)
+
+
+@pytest.mark.parametrize("mode", [api.PRIMAL, api.ADJOINT])
 def test_one_flat_element_among_others(mode):
     """Rows that mix FP64 and fixed-point records, with dM/du of the KS functional."""
     mesh = kuhn_cube(4)
@@ -220,7 +245,6 @@ def test_one_flat_element_among_others(mode):
     c[t[3]] += 0.998 * (c[t[:3]].mean(axis=0) - c[t[3]])
     mesh = Mesh(coords=c, tets=mesh.tets, elem_set=mesh.elem_set, elem_set_names=mesh.elem_set_names, node_sets={},
                 side_sets={})
-    from goal_gb300.mesh import orient_positive
     mesh.tets = orient_positive(c, mesh.tets)
     U = _deformed(mesh, np.eye(3), 1e-6)
     d = api.Disc(mesh)
